@@ -21,10 +21,13 @@
 // the function in double and rounds once, exactly as the strict modules do.
 // So each function returns the double-then-round value for every input.
 //
-// The functions are written once over a lane type F: float (one value;
-// also compiled for the host, with LG_CRF_HOST, for the CPU tests) or
-// float2 (two rays, with the paired f32x2 instructions).  Every operation is
-// a single IEEE round-to-nearest operation (no contraction is left to the
+// exp, log, atan and atanh first take a quick phase (below), whose error is
+// a few 2^-35 to 2^-39 and whose own rounding test leaves one lane in 2^9 to
+// 2^13 to the full phase.  The quick phases are written once over a lane
+// type F: float (one value; also compiled for the host, with LG_CRF_HOST,
+// for the CPU tests) or float2 (two rays, with the paired f32x2
+// instructions); the full phases take one value at a time.  Every operation
+// is a single IEEE round-to-nearest operation (no contraction is left to the
 // compiler).  Tables: lg_crf_tables.cuh, generated by make_crf_tables.py.
 
 #ifdef LG_CRF_HOST
@@ -33,7 +36,7 @@
 #include <cstring>
 #define LG_CRF_DEV static inline
 #define LG_CRF_COLD static
-#define LG_CRF_TABLE(type, name, n) static const type name[n]
+#define LG_CRF_TABLE(name, n) static const unsigned long long name[n]
 struct float2 {
     float x, y;
 };
@@ -43,7 +46,7 @@ struct float4 {
 #else
 #define LG_CRF_DEV static __device__ __forceinline__
 #define LG_CRF_COLD static __device__ __noinline__
-#define LG_CRF_TABLE(type, name, n) __device__ const type name[n]
+#define LG_CRF_TABLE(name, n) __device__ const __align__(16) unsigned long long name[n]
 #endif
 
 // ------------------------------------------------------------- primitives --
@@ -109,13 +112,11 @@ LG_CRF_DEV float crf_add(float a, float b) { return __fadd_rn(a, b); }
 LG_CRF_DEV float crf_sub(float a, float b) { return __fsub_rn(a, b); }
 LG_CRF_DEV float crf_mul(float a, float b) { return __fmul_rn(a, b); }
 LG_CRF_DEV float crf_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-// paired operations: add and fma on f32x2; products lane by lane, because
-// with CUDA 13.0 the assembler fused an f32x2 multiply into the following
-// f32x2 add (scalar round-to-nearest multiplies are never fused), and the
-// double-word steps are written for separately rounded products
+// paired operations on f32x2: add and fma.  (With CUDA 13.0 the assembler
+// fused an f32x2 multiply into a following f32x2 add; see crf_mulx for the
+// products of the quick phases.)
 LG_CRF_DEV float2 crf_add(float2 a, float2 b) { return __fadd2_rn(a, b); }
 LG_CRF_DEV float2 crf_sub(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
-LG_CRF_DEV float2 crf_mul(float2 a, float2 b) { return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y)); }
 LG_CRF_DEV float2 crf_fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 LG_CRF_DEV int crf_bits(float a) { return __float_as_int(a); }
 LG_CRF_DEV float crf_from_bits(int i) { return __int_as_float(i); }
@@ -178,11 +179,24 @@ LG_CRF_DEV void crf_set(float2& v, int i, float s)
     else
         v.x = s;
 }
-template <class T> LG_CRF_DEV T crf_ldg(const T* p) { return __ldg(p); }
+// entry j of a table of float pairs (quads)
+LG_CRF_DEV float2 crf_tab2(const unsigned long long* t, int j) { return __ldg(reinterpret_cast<const float2*>(t) + j); }
+LG_CRF_DEV float4 crf_tab4(const unsigned long long* t, int j) { return __ldg(reinterpret_cast<const float4*>(t) + j); }
 #endif
 
 #ifdef LG_CRF_HOST
-template <class T> LG_CRF_DEV T crf_ldg(const T* p) { return *p; }
+LG_CRF_DEV float2 crf_tab2(const unsigned long long* t, int j)
+{
+    float2 v;
+    std::memcpy(&v, t + j, 8);
+    return v;
+}
+LG_CRF_DEV float4 crf_tab4(const unsigned long long* t, int j)
+{
+    float4 v;
+    std::memcpy(&v, t + 2 * j, 16);
+    return v;
+}
 LG_CRF_DEV float crf_fabsf(float a) { return std::fabs(a); }
 LG_CRF_DEV float crf_copysignf(float a, float b) { return std::copysign(a, b); }
 #else
@@ -245,11 +259,10 @@ LG_CRF_DEV float2 crf_abs(float2 a)
 // means the result.  (lo +- hi 2^-40 from an fma: the product is exact, a
 // power-of-two scaling; for negative hi the two ends swap, which the
 // equality test does not mind.)
-template <class F>
-LG_CRF_DEV void crf_ziv(F hi, F lo, F& z1, F& z2)
+LG_CRF_DEV void crf_ziv(float hi, float lo, float& z1, float& z2)
 {
-    z1 = crf_add(hi, crf_fma(hi, crf_bc<F>(LG_CRF_ZIV), lo));
-    z2 = crf_add(hi, crf_fma(hi, crf_bc<F>(-LG_CRF_ZIV), lo));
+    z1 = crf_add(hi, crf_fma(hi, LG_CRF_ZIV, lo));
+    z2 = crf_add(hi, crf_fma(hi, -LG_CRF_ZIV, lo));
 }
 
 // every lane of v satisfies ok
@@ -300,85 +313,46 @@ LG_CRF_COLD float crf_exp_low(float x, float yh0, float yl0, int m)
 }
 
 // e^r 2^(j/64) as yh + yl for r = rh + rl (|rh| <= ln2/128 + 2^-17, rl to
-// first order) and j, m (k = 64 m + j) from big = k + 1.5 2^23, per lane.
-template <class F>
-LG_CRF_DEV void crf_exp_tail(F big, F rh, F rl, F& yh, F& yl, int (&mm)[2])
+// first order) and j, m (k = 64 m + j) from big = k + 1.5 2^23.
+LG_CRF_DEV void crf_exp_tail(float big, float rh, float rl, float& yh, float& yl, int& m)
 {
-    const F sh = crf_mul(rh, rh);
-    const F sl = crf_fma(rh, rh, crf_neg(sh));
-    const F p3 = crf_fma(rh, crf_bc<F>(0x1.555556p-5f), crf_bc<F>(0x1.555556p-3f));
-    const F h = crf_mul(sh, crf_bc<F>(0.5f));
+    const float sh = crf_mul(rh, rh);
+    const float sl = crf_fma(rh, rh, crf_neg(sh));
+    const float p3 = crf_fma(rh, 0x1.555556p-5f, 0x1.555556p-3f);
+    const float h = crf_mul(sh, 0.5f);
     // first order in rl (up to 2^-22 at large |k|): rl (1 + rh + rh^2/2)
-    const F small = crf_fma(crf_mul(sh, rh), p3, crf_fma(sl, crf_bc<F>(0.5f), crf_fma(h, rl, crf_fma(rh, rl, rl))));
-    const F uh = crf_add(rh, h);  // |rh| >= rh^2 / 2: fast two-sum
-    const F ul = crf_add(crf_sub(h, crf_sub(uh, rh)), small);
-    F th, tl;
-#pragma unroll
-    for (int i = 0; i < crf_lanes<F>::n; ++i) {
-        int j;
-        crf_exp_fields(crf_bits(crf_get(big, i)), j, mm[i]);
-        const float2 T = crf_ldg(lg_crf_exp_tab + j);
-        crf_set(th, i, T.x);
-        crf_set(tl, i, T.y);
-    }
+    const float small = crf_fma(crf_mul(sh, rh), p3, crf_fma(sl, 0.5f, crf_fma(h, rl, crf_fma(rh, rl, rl))));
+    const float uh = crf_add(rh, h);  // |rh| >= rh^2 / 2: fast two-sum
+    const float ul = crf_add(crf_sub(h, crf_sub(uh, rh)), small);
+    int j;
+    crf_exp_fields(crf_bits(big), j, m);
+    const float2 T = crf_tab2(lg_crf_exp_tab, j);
+    const float th = T.x, tl = T.y;
     // T (1 + u) = T + T uh + (T ul + tl uh + tl)
-    const F ph = crf_mul(th, uh);
-    const F pl = crf_fma(th, uh, crf_neg(ph));
-    const F e = crf_add(crf_fma(th, ul, crf_fma(tl, uh, tl)), pl);
+    const float ph = crf_mul(th, uh);
+    const float pl = crf_fma(th, uh, crf_neg(ph));
+    const float e = crf_add(crf_fma(th, ul, crf_fma(tl, uh, tl)), pl);
     yh = crf_add(th, ph);  // |th| >= 1 > |ph|: fast two-sum
     yl = crf_add(crf_sub(ph, crf_sub(yh, th)), e);
 }
 
-// The double-word e^x 2^-m as yh + yl, big = k + 1.5 2^23, and m per lane.
-template <class F>
-LG_CRF_DEV void crf_exp_core(F x, F& big, F& yh, F& yl, int (&mm)[2])
+LG_CRF_DEV float crf_full_exp(float x)
 {
-    const F S = crf_bc<F>(0x1.8p23f);
-    big = crf_fma(x, crf_bc<F>(LG_CRF_EXP_INVL), S);  // k + 1.5 2^23 (|k| < 2^22)
-    const F kf = crf_sub(big, S);
-    const F rh = crf_fma(crf_neg(kf), crf_bc<F>(LG_CRF_EXP_LHI), x);
-    const F rl = crf_mul(crf_neg(kf), crf_bc<F>(LG_CRF_EXP_LLO));
-    crf_exp_tail(big, rh, rl, yh, yl, mm);
-}
-
-template <class F>
-LG_CRF_DEV F lg_crf_exp(F x)
-{
-    F big, yh, yl, z1, z2;
-    int m[2];
-    crf_exp_core(x, big, yh, yl, m);
+    const float S = 0x1.8p23f;
+    const float big = crf_fma(x, LG_CRF_EXP_INVL, S);  // k + 1.5 2^23 (|k| < 2^22)
+    const float kf = crf_sub(big, S);
+    const float rh = crf_fma(crf_neg(kf), LG_CRF_EXP_LHI, x);
+    const float rl = crf_mul(crf_neg(kf), LG_CRF_EXP_LLO);
+    float yh, yl, z1, z2;
+    int m;
+    crf_exp_tail(big, rh, rl, yh, yl, m);
     crf_ziv(yh, yl, z1, z2);
-    F out;
-    // the common case for the whole pair: x in [-87, 88] (a normal result,
-    // so m >= -125 or m = -126 with z1 >= 1) and the rounding decided
-    bool ok[2];
-#pragma unroll
-    for (int i = 0; i < crf_lanes<F>::n; ++i) {
-        const float xi = crf_get(x, i);
-        ok[i] = xi >= -87.0f && xi <= 88.0f && crf_get(z1, i) == crf_get(z2, i);
+    if (x <= 88.0f && x > LG_CRF_EXP_ZERO) {
+        if (m >= -125 || (m == -126 && z1 >= 1.0f))
+            return z1 == z2 ? crf_from_bits(crf_add_exp(crf_bits(z1), m)) : crf_slow_exp(x);
+        return crf_exp_low(x, yh, yl, m);
     }
-    if (crf_all<F>(ok)) {
-#pragma unroll
-        for (int i = 0; i < crf_lanes<F>::n; ++i)
-            crf_set(out, i, crf_from_bits(crf_add_exp(crf_bits(crf_get(z1, i)), m[i])));
-        return out;
-    }
-#pragma unroll
-    for (int i = 0; i < crf_lanes<F>::n; ++i) {
-        const float xi = crf_get(x, i);
-        float r;
-        if (xi <= 88.0f && xi > LG_CRF_EXP_ZERO) {
-            const float a = crf_get(z1, i);
-            if (m[i] >= -125 || (m[i] == -126 && a >= 1.0f))
-                r = a == crf_get(z2, i) ? crf_from_bits(crf_add_exp(crf_bits(a), m[i])) : crf_slow_exp(xi);
-            else
-                r = crf_exp_low(xi, crf_get(yh, i), crf_get(yl, i), m[i]);
-        } else {
-            r = xi <= LG_CRF_EXP_ZERO ? 0.0f : crf_slow_exp(xi);  // NaN, x > 88: in double
-        }
-        crf_set(out, i, r);
-    }
-    return out;
+    return x <= LG_CRF_EXP_ZERO ? 0.0f : crf_slow_exp(x);  // NaN, x > 88: in double
 }
 
 // ---------------------------------------------------------------------- log --
@@ -386,16 +360,15 @@ LG_CRF_DEV F lg_crf_exp(F x)
 // (1/3 - r/4 + r^2/5), the square exact; truncation r^6/6 (relative 2^-52
 // where the result is r itself), the cubic term in float (relative to r,
 // 3 roundings of a term below 2^-21.6: 2^-44).  Out: uh + ul.
-template <class F>
-LG_CRF_DEV void crf_log1p_dw(F rh, F rl, F& uh, F& ul)
+LG_CRF_DEV void crf_log1p_dw(float rh, float rl, float& uh, float& ul)
 {
-    const F sh = crf_mul(rh, rh);
-    const F sl = crf_fma(rh, rh, crf_neg(sh));
-    const F P = crf_fma(crf_fma(rh, crf_bc<F>(0x1.99999ap-3f), crf_bc<F>(-0.25f)), rh, crf_bc<F>(0x1.555556p-2f));
-    const F t = crf_mul(crf_mul(sh, rh), P);
+    const float sh = crf_mul(rh, rh);
+    const float sl = crf_fma(rh, rh, crf_neg(sh));
+    const float P = crf_fma(crf_fma(rh, 0x1.99999ap-3f, -0.25f), rh, 0x1.555556p-2f);
+    const float t = crf_mul(crf_mul(sh, rh), P);
     // r_lo - r_h r_lo - s_lo / 2 + t
-    const F small = crf_add(crf_fma(crf_neg(rh), rl, rl), crf_fma(sl, crf_bc<F>(-0.5f), t));
-    const F h = crf_mul(sh, crf_bc<F>(-0.5f));
+    const float small = crf_add(crf_fma(crf_neg(rh), rl, rl), crf_fma(sl, -0.5f, t));
+    const float h = crf_mul(sh, -0.5f);
     uh = crf_add(rh, h);  // |rh| >= rh^2 / 2: fast two-sum
     ul = crf_add(crf_sub(h, crf_sub(uh, rh)), small);
 }
@@ -408,72 +381,55 @@ LG_CRF_DEV void crf_log1p_dw(F rh, F rl, F& uh, F& ul)
 // relative accuracy.  Sum: e ln2 as an exact product pair plus e LN2_LO,
 // then two fast two-sums (|e ln2| >= |ln c_j| >= |log1p(r)| or the larger
 // term is zero).  Out: hi + lo.
-template <class F, bool DW>
-LG_CRF_DEV void crf_log_dw(F uh, F ul, F& hi, F& lo)
+template <bool DW>
+LG_CRF_DEV void crf_log_dw(float uh, float ul, float& hi, float& lo)
 {
-    F m, c, Lh, Ll, ef, ml;
-#pragma unroll
-    for (int i = 0; i < crf_lanes<F>::n; ++i) {
-        int e, j, mb;
-        crf_log_fields(crf_bits(crf_get(uh, i)), e, j, mb);
-        crf_set(m, i, crf_from_bits(mb));
-        const float4 T = crf_ldg(lg_crf_log_tab + j);
-        crf_set(c, i, T.x);
-        crf_set(Lh, i, T.y);
-        crf_set(Ll, i, T.z);
-        // e as float: e + 1.5 2^23 has the bits 0x4b400000 + e
-        crf_set(ef, i, crf_from_bits(0x4b400000 + e) - 0x1.8p23f);
-        if (DW) crf_set(ml, i, crf_get(ul, i) * crf_from_bits(crf_pow2_bits(-e)));  // exact: ul 2^-e
-    }
-    const F ph = crf_mul(m, c);
-    const F pl = crf_fma(m, c, crf_neg(ph));
-    F rh = crf_sub(ph, crf_bc<F>(1.0f));  // exact
-    F rl;
+    int e, j, mb;
+    crf_log_fields(crf_bits(uh), e, j, mb);
+    const float m = crf_from_bits(mb);
+    const float4 T = crf_tab4(lg_crf_log_tab, j);
+    const float c = T.x, Lh = T.y, Ll = T.z;
+    // e as float: e + 1.5 2^23 has the bits 0x4b400000 + e
+    const float ef = crf_sub(crf_from_bits(0x4b400000 + e), 0x1.8p23f);
+    const float ph = crf_mul(m, c);
+    const float pl = crf_fma(m, c, crf_neg(ph));
+    float rh = crf_sub(ph, 1.0f);  // exact
+    float rl;
     if (DW) {
         // + m_lo c, then renormalise (two-sum: m_lo can exceed rh)
-        const F q = crf_fma(ml, c, pl);
-        const F s = crf_add(rh, q);
-        const F bb = crf_sub(s, rh);
+        const float ml = crf_mul(ul, crf_from_bits(crf_pow2_bits(-e)));  // exact: ul 2^-e
+        const float q = crf_fma(ml, c, pl);
+        const float s = crf_add(rh, q);
+        const float bb = crf_sub(s, rh);
         rl = crf_add(crf_sub(rh, crf_sub(s, bb)), crf_sub(q, bb));
         rh = s;
     } else {
         // renormalise: pl (up to 2^-25) would otherwise dominate the
         // rounding errors of small r (fast two-sum: rh = 0 or |rh| >= 2^-24)
-        const F s = crf_add(rh, pl);
+        const float s = crf_add(rh, pl);
         rl = crf_sub(pl, crf_sub(s, rh));
         rh = s;
     }
-    F vh, vl;
+    float vh, vl;
     crf_log1p_dw(rh, rl, vh, vl);
-    const F a1 = crf_mul(ef, crf_bc<F>(LG_CRF_LN2_HI));
-    const F a1l = crf_fma(ef, crf_bc<F>(LG_CRF_LN2_HI), crf_neg(a1));
-    const F a1l2 = crf_mul(ef, crf_bc<F>(LG_CRF_LN2_LO));
-    const F s1 = crf_add(a1, Lh);
-    const F e1 = crf_sub(Lh, crf_sub(s1, a1));
+    const float a1 = crf_mul(ef, LG_CRF_LN2_HI);
+    const float a1l = crf_fma(ef, LG_CRF_LN2_HI, crf_neg(a1));
+    const float a1l2 = crf_mul(ef, LG_CRF_LN2_LO);
+    const float s1 = crf_add(a1, Lh);
+    const float e1 = crf_sub(Lh, crf_sub(s1, a1));
     hi = crf_add(s1, vh);
-    const F e2 = crf_sub(vh, crf_sub(hi, s1));
+    const float e2 = crf_sub(vh, crf_sub(hi, s1));
     lo = crf_add(crf_add(e1, e2), crf_add(crf_add(a1l, a1l2), crf_add(Ll, vl)));
 }
 
-template <class F>
-LG_CRF_DEV F lg_crf_log(F x)
+LG_CRF_DEV float crf_full_log(float x)
 {
-    F hi, lo, z1, z2;
-    crf_log_dw<F, false>(x, x, hi, lo);
+    float hi, lo, z1, z2;
+    crf_log_dw<false>(x, x, hi, lo);
     crf_ziv(hi, lo, z1, z2);
     // normal, positive, finite x with the rounding decided; zero, negative,
     // subnormal, infinite and NaN x in double
-    bool ok[2];
-#pragma unroll
-    for (int i = 0; i < crf_lanes<F>::n; ++i) {
-        const float xi = crf_get(x, i);
-        ok[i] = xi >= 0x1p-126f && xi <= 0x1.fffffep127f && crf_get(z1, i) == crf_get(z2, i);
-    }
-    if (crf_all<F>(ok)) return z1;
-    F out;
-#pragma unroll
-    for (int i = 0; i < crf_lanes<F>::n; ++i) crf_set(out, i, ok[i] ? crf_get(z1, i) : crf_slow_log(crf_get(x, i)));
-    return out;
+    return x >= 0x1p-126f && x <= 0x1.fffffep127f && z1 == z2 ? z1 : crf_slow_log(x);
 }
 
 // --------------------------------------------------------------------- atan --
@@ -486,96 +442,53 @@ LG_CRF_DEV F lg_crf_log(F x)
 // cubic term in float (relative to delta 2^-44).  For a > 1 the result is
 // pi/2 - that.  Error about 2^-44.
 // atan t for t = th + tl in [0, 1] (tl a few ulp of th at most) as s1 + lo.
-template <class F>
-LG_CRF_DEV void crf_atan_core(F th, F tl, F& s1, F& lo)
+LG_CRF_DEV void crf_atan_core(float th, float tl, float& s1, float& lo)
 {
-    F rd, Ah, Al;
-    const F S = crf_bc<F>(0x1.8p23f);
-    const F big = crf_fma(th, crf_bc<F>(512.0f), S);
-    const F tj = crf_mul(crf_sub(big, S), crf_bc<F>(0x1p-9f));
-#pragma unroll
-    for (int i = 0; i < crf_lanes<F>::n; ++i) {
-        int j = crf_bits(crf_get(big, i)) - 0x4b400000;
-        j = j < 0 ? 0 : (j > 512 ? 512 : j);  // (in range for every finite t in [0, 1])
-        const float2 A = crf_ldg(lg_crf_atan_tab + j);
-        crf_set(Ah, i, A.x);
-        crf_set(Al, i, A.y);
-    }
-    const F nh = crf_sub(th, tj);  // exact
-    const F qh = crf_mul(th, tj);
-    const F ql = crf_fma(th, tj, crf_neg(qh));
-    const F dh = crf_add(crf_bc<F>(1.0f), qh);  // 1 >= qh: fast two-sum
-    const F dl = crf_add(crf_sub(qh, crf_sub(dh, crf_bc<F>(1.0f))), crf_fma(tl, tj, ql));
-#pragma unroll
-    for (int i = 0; i < crf_lanes<F>::n; ++i) crf_set(rd, i, crf_rcp(crf_get(dh, i)));  // dh in [1, 2]
-    const F d0 = crf_mul(nh, rd);
-    const F res = crf_add(crf_fma(crf_neg(d0), dh, nh), crf_fma(crf_neg(d0), dl, tl));
-    const F d1 = crf_mul(res, rd);
-    const F s = crf_mul(d0, d0);
-    const F P = crf_fma(s, crf_bc<F>(0x1.99999ap-3f), crf_bc<F>(-0x1.555556p-2f));
-    const F cub = crf_mul(crf_mul(s, d0), P);
+    const float S = 0x1.8p23f;
+    const float big = crf_fma(th, 512.0f, S);
+    const float tj = crf_mul(crf_sub(big, S), 0x1p-9f);
+    int j = crf_bits(big) - 0x4b400000;
+    j = j < 0 ? 0 : (j > 512 ? 512 : j);  // (in range for every finite t in [0, 1])
+    const float2 A = crf_tab2(lg_crf_atan_tab, j);
+    const float Ah = A.x, Al = A.y;
+    const float nh = crf_sub(th, tj);  // exact
+    const float qh = crf_mul(th, tj);
+    const float ql = crf_fma(th, tj, crf_neg(qh));
+    const float dh = crf_add(1.0f, qh);  // 1 >= qh: fast two-sum
+    const float dl = crf_add(crf_sub(qh, crf_sub(dh, 1.0f)), crf_fma(tl, tj, ql));
+    const float rd = crf_rcp(dh);  // dh in [1, 2]
+    const float d0 = crf_mul(nh, rd);
+    const float res = crf_add(crf_fma(crf_neg(d0), dh, nh), crf_fma(crf_neg(d0), dl, tl));
+    const float d1 = crf_mul(res, rd);
+    const float s = crf_mul(d0, d0);
+    const float P = crf_fma(s, 0x1.99999ap-3f, -0x1.555556p-2f);
+    const float cub = crf_mul(crf_mul(s, d0), P);
     s1 = crf_add(Ah, d0);  // |atan t_j| >= |delta| or t_j = 0
-    const F e1 = crf_sub(d0, crf_sub(s1, Ah));
+    const float e1 = crf_sub(d0, crf_sub(s1, Ah));
     lo = crf_add(crf_add(e1, Al), crf_add(d1, cub));
 }
 
-template <class F>
-LG_CRF_DEV F lg_crf_atan(F z)
+LG_CRF_DEV float crf_full_atan(float z)
 {
-    const F a = crf_abs(z);
-    F th = a, tl = crf_bc<F>(0.0f);
-    bool inv[2];
-    bool any_inv = false;
-#pragma unroll
-    for (int i = 0; i < crf_lanes<F>::n; ++i) {
-        inv[i] = crf_get(a, i) > 1.0f;
-        any_inv = any_inv || inv[i];
+    const float a = crf_abs(z);
+    const bool inv = a > 1.0f;
+    float th = a, tl = 0.0f;
+    if (inv) {  // 1/a (a > 2^126 flushes to 0; atan is then RN(pi/2))
+        th = crf_rcp(a);
+        tl = crf_mul(crf_fma(crf_neg(th), a, 1.0f), th);
     }
-    // the reciprocal and pi/2 - ... only where a lane needs them (the SIE
-    // family's arguments rarely exceed 1)
-    if (any_inv) {
-        F r0;
-#pragma unroll
-        for (int i = 0; i < crf_lanes<F>::n; ++i)  // 1/a for a > 1 (a > 2^126 flushes to 0; atan is then RN(pi/2))
-            crf_set(r0, i, inv[i] ? crf_rcp(crf_get(a, i)) : 1.0f);
-        const F rho = crf_fma(crf_neg(r0), a, crf_bc<F>(1.0f));
-        const F r1 = crf_mul(rho, r0);
-#pragma unroll
-        for (int i = 0; i < crf_lanes<F>::n; ++i) {
-            crf_set(th, i, inv[i] ? crf_get(r0, i) : crf_get(a, i));
-            crf_set(tl, i, inv[i] ? crf_get(r1, i) : 0.0f);
-        }
+    float hi, lo, z1, z2;
+    crf_atan_core(th, tl, hi, lo);
+    if (inv) {  // pi/2 - (hi + lo)
+        const float ph = crf_sub(LG_CRF_PIO2_HI, hi);
+        const float pe = crf_sub(crf_sub(LG_CRF_PIO2_HI, ph), hi);
+        lo = crf_add(pe, crf_sub(LG_CRF_PIO2_LO, lo));
+        hi = ph;
     }
-    F s1, lo;
-    crf_atan_core(th, tl, s1, lo);
-    F hi2 = s1, lo2 = lo;
-    if (any_inv) {  // pi/2 - (s1 + lo)
-        const F ph = crf_sub(crf_bc<F>(LG_CRF_PIO2_HI), s1);
-        const F pe = crf_sub(crf_sub(crf_bc<F>(LG_CRF_PIO2_HI), ph), s1);
-        const F plo = crf_add(pe, crf_sub(crf_bc<F>(LG_CRF_PIO2_LO), lo));
-#pragma unroll
-        for (int i = 0; i < crf_lanes<F>::n; ++i) {
-            crf_set(hi2, i, inv[i] ? crf_get(ph, i) : crf_get(s1, i));
-            crf_set(lo2, i, inv[i] ? crf_get(plo, i) : crf_get(lo, i));
-        }
-    }
-    F z1, z2;
-    crf_ziv(hi2, lo2, z1, z2);
+    crf_ziv(hi, lo, z1, z2);
     // finite z with the rounding decided; infinite and NaN z in double.  The
     // sign of z on |result| (z = +-0 gives +-0: the result is 0 there).
-    bool ok[2];
-    F out;
-#pragma unroll
-    for (int i = 0; i < crf_lanes<F>::n; ++i) {
-        const float zi = crf_get(z, i);
-        ok[i] = crf_fabsf(zi) <= 0x1.fffffep127f && crf_get(z1, i) == crf_get(z2, i);
-        crf_set(out, i, crf_copysignf(crf_get(z1, i), zi));
-    }
-    if (crf_all<F>(ok)) return out;
-#pragma unroll
-    for (int i = 0; i < crf_lanes<F>::n; ++i)
-        if (!ok[i]) crf_set(out, i, crf_slow_atan(crf_get(z, i)));
-    return out;
+    return a <= 0x1.fffffep127f && z1 == z2 ? crf_copysignf(z1, z) : crf_slow_atan(z);
 }
 
 // -------------------------------------------------------------------- atanh --
@@ -592,92 +505,340 @@ LG_CRF_DEV F lg_crf_atan(F z)
 //    step), 1 + w as a two-sum, then the double-word logarithm: 1 + w
 //    carries about 2^-49 absolute error, 2^-46 of the result here.
 // The SIE family's arguments stay below sqrt(1 - q^2), so its rays take the
-// first formula unless q < 0.44; each branch runs only where a lane of the
-// pair needs it.
+// first formula unless q < 0.44.
+LG_CRF_DEV float crf_full_atanh(float v)
+{
+    const float a = crf_abs(v);
+    const float one = 1.0f;
+    float hi, lo, z1, z2;
+    if (a <= 0.9f) {
+        const float S = 0x1.8p23f;
+        const float big = crf_fma(a, 512.0f, S);
+        const float tj = crf_mul(crf_sub(big, S), 0x1p-9f);
+        const float2 A = crf_tab2(lg_crf_atanh_tab, crf_bits(big) - 0x4b400000);
+        const float Ah = A.x, Al = A.y;
+        const float nh = crf_sub(a, tj);  // exact
+        const float qh = crf_mul(a, tj);
+        const float ql = crf_fma(a, tj, crf_neg(qh));
+        const float dh = crf_sub(one, qh);  // 1 >= qh: fast two-sum
+        const float dl = crf_sub(crf_sub(crf_sub(one, dh), qh), ql);
+        const float rd = crf_rcp(dh);  // dh in [0.19, 1]
+        const float d0 = crf_mul(nh, rd);
+        const float res = crf_fma(crf_neg(d0), dl, crf_fma(crf_neg(d0), dh, nh));
+        const float d1 = crf_mul(res, rd);
+        const float s = crf_mul(d0, d0);
+        const float P = crf_fma(s, 0x1.99999ap-3f, 0x1.555556p-2f);
+        const float cub = crf_mul(crf_mul(s, d0), P);
+        hi = crf_add(Ah, d0);  // |atanh t_j| >= |delta| or t_j = 0: fast two-sum
+        const float e1 = crf_sub(d0, crf_sub(hi, Ah));
+        lo = crf_add(crf_add(e1, Al), crf_add(d1, cub));
+    } else {
+        const float dh = crf_sub(one, a);
+        const float dl = crf_sub(crf_sub(one, dh), a);  // exact (1 >= a)
+        const float n = crf_add(a, a);
+        const float rd = crf_rcp(dh);  // dh >= 2^-24
+        const float w0 = crf_mul(n, rd);
+        const float res = crf_fma(crf_neg(w0), dl, crf_fma(crf_neg(w0), dh, n));
+        const float w1 = crf_mul(res, rd);
+        // 1 + w0 (two-sum: w0 may exceed 1), + w1
+        const float uh = crf_add(one, w0);
+        const float bb = crf_sub(uh, one);
+        const float ul = crf_add(crf_add(crf_sub(one, crf_sub(uh, bb)), crf_sub(w0, bb)), w1);
+        crf_log_dw<true>(uh, ul, hi, lo);
+        hi = crf_mul(hi, 0.5f);
+        lo = crf_mul(lo, 0.5f);
+    }
+    crf_ziv(hi, lo, z1, z2);
+    // |v| < 1 with the rounding decided; |v| >= 1 and NaN v in double.  The
+    // sign of v on |result| (v = +-0 gives +-0).
+    return a < 1.0f && z1 == z2 ? crf_copysignf(z1, v) : crf_slow_atanh(v);
+}
+
+// ------------------------------------------------------------ quick phases --
+// exp, log, atan and atanh as the exact render calls them: a first phase of
+// 16-24 operations whose error is far below half a float ulp, Ziv's test on
+// its interval, and the functions above (out of line) for the lanes it
+// leaves undecided.  All F operations run on both lanes of a pair at once.
+//
+// products that enter only terms whose rounding errors the interval covers:
+// on pairs the packed multiply (contracting it into a following add would
+// only lower the error)
+LG_CRF_DEV float crf_mulx(float a, float b) { return crf_mul(a, b); }
+#ifndef LG_CRF_HOST
+LG_CRF_DEV float2 crf_mulx(float2 a, float2 b) { return __fmul2_rn(a, b); }
+#endif
+#ifndef LG_CRF_REST_COUNT
+#define LG_CRF_REST_COUNT()
+#endif
+LG_CRF_COLD float crf_rest_exp(float x)
+{
+    LG_CRF_REST_COUNT();
+    if (x <= LG_CRF_EXP_ZERO) return 0.0f;  // the wings of compact profiles
+    return crf_full_exp(x);
+}
+LG_CRF_COLD float crf_rest_log(float x) { LG_CRF_REST_COUNT(); return crf_full_log(x); }
+LG_CRF_COLD float crf_rest_atan(float x) { LG_CRF_REST_COUNT(); return crf_full_atan(x); }
+LG_CRF_COLD float crf_rest_atanh(float x) { LG_CRF_REST_COUNT(); return crf_full_atanh(x); }
+
+// integer fields, in inline PTX as above:
+//   exp: z 2^m for k = 1024 m + j, big's bits = bits(1.5 2^23) + k (the
+//        constant's bits leave the word in the shift)
+//   log: the mantissa in [1, 2) and the biased exponent times 2^23
+#ifdef LG_CRF_HOST
+LG_CRF_DEV int crf_qexp_scale(int zbits, int bits) { return (int)((unsigned)zbits + ((unsigned)(bits & ~1023) << 13)); }
+LG_CRF_DEV void crf_qlog_fields(int b, int& mb, int& te)
+{
+    mb = (b & 0x007fffff) | 0x3f800000;
+    te = b & 0x7f800000;
+}
+#else
+LG_CRF_DEV int crf_qexp_scale(int zbits, int bits)
+{
+    int r;
+    asm("{\n.reg .s32 t;\nand.b32 t, %2, 0xfffffc00;\nshl.b32 t, t, 13;\nadd.s32 %0, %1, t;\n}"
+        : "=r"(r)
+        : "r"(zbits), "r"(bits));
+    return r;
+}
+LG_CRF_DEV void crf_qlog_fields(int b, int& mb, int& te)
+{
+    asm("{\n.reg .b32 t;\nand.b32 t, %2, 0x007fffff;\nor.b32 %0, t, 0x3f800000;\nand.b32 %1, %2, 0x7f800000;\n}"
+        : "=r"(mb), "=r"(te)
+        : "r"(b));
+}
+#endif
+
+// e^x, |x| <= 87: x = k ln2/1024 + r, |r| <= 2^-11.5, k = 1024 m + j; with
+// T = 2^(j/1024) = th + tl, e^x 2^-m = th + (th rh + (th (rl + rh (rh/2 + rl)) + tl
+// + tl rh)): rh = x - k L_hi exact, rl = -k L_lo.  Absolute error of the sum before its
+// rounding: that of the inner sum (2^-35), r^3/6 (2^-36.2 with T < 2), the
+// rest below 2^-41; the table's second entry holds tl + D with D = 1.625
+// 2^-35, the interval's half-width.
+template <class F>
+LG_CRF_DEV F lg_crf_exp(F x)
+{
+    const F big = crf_fma(x, crf_bc<F>(LG_CRF_QEXP_INVL), crf_bc<F>(0x1.8p23f));
+    const F kf = crf_add(big, crf_bc<F>(-0x1.8p23f));
+    const F rh = crf_fma(kf, crf_bc<F>(-LG_CRF_QEXP_LHI), x);
+    const F rl = crf_mulx(kf, crf_bc<F>(-LG_CRF_QEXP_LLO));
+    const F sm = crf_fma(rh, crf_fma(rh, crf_bc<F>(0.5f), rl), rl);
+    F th, tl;
+#pragma unroll
+    for (int i = 0; i < crf_lanes<F>::n; ++i) {
+        const float2 T = crf_tab2(lg_crf_qexp_tab, (crf_bits(crf_get(big, i)) & 1023));
+        crf_set(th, i, T.x);
+        crf_set(tl, i, T.y);
+    }
+    const F w1 = crf_fma(th, sm, crf_fma(tl, rh, tl));
+    const F w2 = crf_add(w1, crf_bc<F>(-0x1.ap-34f));
+    const F z1 = crf_add(th, crf_fma(th, rh, w1));
+    const F z2 = crf_add(th, crf_fma(th, rh, w2));
+    F out;
+    bool ok[2];
+#pragma unroll
+    for (int i = 0; i < crf_lanes<F>::n; ++i) {
+        ok[i] = crf_fabsf(crf_get(x, i)) <= 87.0f && crf_get(z1, i) == crf_get(z2, i);
+        crf_set(out, i, crf_from_bits(crf_qexp_scale(crf_bits(crf_get(z1, i)), crf_bits(crf_get(big, i)))));
+    }
+    if (!crf_all<F>(ok)) {
+#pragma unroll
+        for (int i = 0; i < crf_lanes<F>::n; ++i)
+            if (!ok[i]) crf_set(out, i, crf_rest_exp(crf_get(x, i)));
+    }
+    return out;
+}
+
+// ln x, x normal: x = 2^e m, m in [1, 2), c = 1/m cut to 11 significant bits
+// (from the reciprocal estimate; any estimate serves), so that r = m c - 1
+// (|r| <= 2^-10) is exact; ln x = (e ln2_hi + Lh) + (r + (r^2 (r/3 - 1/2) + e
+// ln2_lo + Ll)) with -ln c = Lh + Ll, Lh and ln2_hi multiples of 2^-17: the
+// first sum is exact.  Absolute error: the sum with r (2^-34 at most, the
+// rest of it reaching 2^-11), e ln2_lo + Ll (2^-36), r^4/4 (2^-42); D =
+// 1.375 2^-34.  Results near 0 are left to the full phase.
+template <class F>
+LG_CRF_DEV F lg_crf_log(F x)
+{
+    F m, c, Lh, Ll, ef;
+#pragma unroll
+    for (int i = 0; i < crf_lanes<F>::n; ++i) {
+        int mb, te;
+        crf_qlog_fields(crf_bits(crf_get(x, i)), mb, te);
+        const int cb = crf_bits(crf_rcp(crf_from_bits(mb))) & (int)0xffffe000;
+        const float2 T = crf_tab2(lg_crf_qlog_tab, (int)((unsigned)cb >> 13) - (0x3effe000 >> 13));
+        crf_set(m, i, crf_from_bits(mb));
+        crf_set(c, i, crf_from_bits(cb));
+        crf_set(Lh, i, T.x);
+        crf_set(Ll, i, T.y);
+        crf_set(ef, i, (float)te);  // exact
+    }
+    const F r = crf_fma(m, c, crf_bc<F>(-1.0f));
+    const F e = crf_add(ef, crf_bc<F>(-127.0f * 0x1p23f));
+    const F s1 = crf_fma(e, crf_bc<F>(LG_CRF_QLN2_HI), Lh);
+    const F lo = crf_fma(e, crf_bc<F>(LG_CRF_QLN2_LO), Ll);
+    const F w = crf_fma(r, crf_bc<F>(0x1.555556p-2f), crf_bc<F>(-0.5f));
+    const F t = crf_fma(crf_mulx(r, r), w, lo);
+    const F z1 = crf_add(s1, crf_add(r, crf_add(t, crf_bc<F>(0x1.6p-34f))));
+    const F z2 = crf_add(s1, crf_add(r, crf_add(t, crf_bc<F>(-0x1.6p-34f))));
+    F out = z1;
+    bool ok[2];
+#pragma unroll
+    for (int i = 0; i < crf_lanes<F>::n; ++i)
+        ok[i] = (unsigned)crf_bits(crf_get(x, i)) - 0x00800000u < 0x7f000000u && crf_get(z1, i) == crf_get(z2, i);
+    if (!crf_all<F>(ok)) {
+#pragma unroll
+        for (int i = 0; i < crf_lanes<F>::n; ++i)
+            if (!ok[i]) crf_set(out, i, crf_rest_log(crf_get(x, i)));
+    }
+    return out;
+}
+
+// both ends of the interval hi + lo -+ |hi| 2^-38, rounded
+template <class F>
+LG_CRF_DEV void crf_quick_ziv(F hi, F lo, F& z1, F& z2)
+{
+    z1 = crf_add(hi, crf_fma(hi, crf_bc<F>(0x1p-38f), lo));
+    z2 = crf_add(hi, crf_fma(hi, crf_bc<F>(-0x1p-38f), lo));
+}
+
+// atan t for t in [0, 1]: with t_j = j/512 nearest t, n = t - t_j and d = n /
+// (1 + t_j^2) (the denominator exact), atan t = atan t_j + d - t_j d^2 + (t_j^2
+// - 1/3) d^3 + O(d^4 t_j) (Taylor's series in d; |d| <= 2^-10, the omitted
+// term 2^-40 of the result).  d as a double word from the reciprocal estimate
+// and one correction.  The series' signs are kept negated (nd = -d) so that
+// no operand needs a negation.
+template <class F, bool DW>
+LG_CRF_DEV void crf_quick_atan(F t, F tl, F& s1, F& lo)
+{
+    const F big = crf_add(t, crf_bc<F>(0x1.8p14f));  // t to the nearest 2^-9
+    const F tj = crf_add(big, crf_bc<F>(-0x1.8p14f));
+    F Ah, Al, nr;
+#pragma unroll
+    for (int i = 0; i < crf_lanes<F>::n; ++i) {
+        const float2 A = crf_tab2(lg_crf_atan_tab, (crf_bits(crf_get(big, i)) - 0x46c00000));
+        crf_set(Ah, i, A.x);
+        crf_set(Al, i, A.y);
+    }
+    const F n = crf_fma(tj, crf_bc<F>(-1.0f), t);
+    const F s = crf_fma(tj, tj, crf_bc<F>(1.0f));
+#pragma unroll
+    for (int i = 0; i < crf_lanes<F>::n; ++i) crf_set(nr, i, crf_rcp(-crf_get(s, i)));
+    const F nd = crf_mulx(n, nr);
+    F res = crf_fma(nd, s, n);
+    if (DW) res = crf_add(res, tl);
+    F nd1 = crf_mulx(res, nr);
+    if (DW) nd1 = crf_fma(crf_add(nd1, nd1), crf_mulx(tj, nd), nd1);  // the square's cross term with tl
+    const F P = crf_fma(crf_add(s, crf_bc<F>(-0x1.555556p+0f)), nd, tj);
+    const F nc = crf_fma(crf_mulx(nd, nd), P, nd1);
+    s1 = crf_fma(nd, crf_bc<F>(-1.0f), Ah);
+    const F ne = crf_add(nd, crf_fma(Ah, crf_bc<F>(-1.0f), s1));
+    lo = crf_fma(crf_add(ne, nc), crf_bc<F>(-1.0f), Al);
+}
+// pairs with a lane above 1 (or NaN): t = 1/a there as a double word (a >
+// 2^126 flushes it to 0: the result is RN(pi/2)), and pi/2 - atan t
+template <class F>
+LG_CRF_COLD F crf_wide_atan(F z)
+{
+    const F a = crf_abs(z);
+    F r0, th, tl, s1, lo, z1, z2, out;
+#pragma unroll
+    for (int i = 0; i < crf_lanes<F>::n; ++i) crf_set(r0, i, crf_get(a, i) > 1.0f ? crf_rcp(crf_get(a, i)) : 1.0f);
+    const F r1 = crf_mulx(crf_fma(crf_neg(r0), a, crf_bc<F>(1.0f)), r0);
+#pragma unroll
+    for (int i = 0; i < crf_lanes<F>::n; ++i) {
+        const bool inv = crf_get(a, i) > 1.0f;
+        // (NaN takes 1 here and the double evaluation below)
+        crf_set(th, i, inv || !(crf_get(a, i) <= 1.0f) ? crf_get(r0, i) : crf_get(a, i));
+        crf_set(tl, i, inv ? crf_get(r1, i) : 0.0f);
+    }
+    crf_quick_atan<F, true>(th, tl, s1, lo);
+    const F ph = crf_fma(s1, crf_bc<F>(-1.0f), crf_bc<F>(LG_CRF_PIO2_HI));
+    const F pe = crf_sub(crf_sub(crf_bc<F>(LG_CRF_PIO2_HI), ph), s1);
+    const F pl = crf_add(pe, crf_sub(crf_bc<F>(LG_CRF_PIO2_LO), lo));
+#pragma unroll
+    for (int i = 0; i < crf_lanes<F>::n; ++i)
+        if (crf_get(a, i) > 1.0f) {
+            crf_set(s1, i, crf_get(ph, i));
+            crf_set(lo, i, crf_get(pl, i));
+        }
+    crf_quick_ziv(s1, lo, z1, z2);
+#pragma unroll
+    for (int i = 0; i < crf_lanes<F>::n; ++i) {
+        const float zi = crf_get(z, i);
+        const bool ok = crf_fabsf(zi) <= 0x1.fffffep127f && crf_get(z1, i) == crf_get(z2, i);
+        crf_set(out, i, ok ? crf_copysignf(crf_get(z1, i), zi) : crf_rest_atan(zi));
+    }
+    return out;
+}
+template <class F>
+LG_CRF_DEV F lg_crf_atan(F z)
+{
+    const F a = crf_abs(z);
+    bool in = true;
+#pragma unroll
+    for (int i = 0; i < crf_lanes<F>::n; ++i) in = in && crf_get(a, i) <= 1.0f;
+    if (!in) return crf_wide_atan(z);
+    F s1, lo, z1, z2, out;
+    crf_quick_atan<F, false>(a, a, s1, lo);
+    crf_quick_ziv(s1, lo, z1, z2);
+    bool ok[2];
+#pragma unroll
+    for (int i = 0; i < crf_lanes<F>::n; ++i) {
+        ok[i] = crf_get(z1, i) == crf_get(z2, i);
+        crf_set(out, i, crf_copysignf(crf_get(z1, i), crf_get(z, i)));
+    }
+    if (!crf_all<F>(ok)) {
+#pragma unroll
+        for (int i = 0; i < crf_lanes<F>::n; ++i)
+            if (!ok[i]) crf_set(out, i, crf_rest_atan(crf_get(z, i)));
+    }
+    return out;
+}
+
+// atanh v, a = |v| <= 0.9: with t_j = j/512 nearest a and n = a - t_j, atanh a =
+// atanh t_j + atanh d, d = n / (1 - a t_j), 1 - a t_j = (1 - t_j^2) - n t_j as a
+// double word (both terms exact), d as a double word from the reciprocal
+// estimate and one correction, atanh d = d + d^3/3 (|d| <= 2^-7.6 at a = 0.9:
+// d^5/5 is 2^-40.8 of the result).
 template <class F>
 LG_CRF_DEV F lg_crf_atanh(F v)
 {
     const F a = crf_abs(v);
-    const F one = crf_bc<F>(1.0f);
-    bool tab[2];
-    bool any_tab = false, any_large = false;
+    const F big = crf_add(a, crf_bc<F>(0x1.8p14f));
+    const F tj = crf_add(big, crf_bc<F>(-0x1.8p14f));
+    F Ah, Al, rd;
 #pragma unroll
     for (int i = 0; i < crf_lanes<F>::n; ++i) {
-        tab[i] = crf_get(a, i) <= 0.9f;
-        any_tab = any_tab || tab[i];
-        any_large = any_large || !tab[i];
+        // (the mask keeps arguments outside the range inside the table)
+        const float2 A = crf_tab2(lg_crf_atanh_tab, (crf_bits(crf_get(big, i)) & 511));
+        crf_set(Ah, i, A.x);
+        crf_set(Al, i, A.y);
     }
-    F hs = a, ls = a, hl = a, ll = a;
-    if (any_tab) {
-        const F S = crf_bc<F>(0x1.8p23f);
-        const F big = crf_fma(a, crf_bc<F>(512.0f), S);
-        const F tj = crf_mul(crf_sub(big, S), crf_bc<F>(0x1p-9f));
-        F Ah, Al, rd;
+    const F n = crf_fma(tj, crf_bc<F>(-1.0f), a);
+    const F nD = crf_fma(tj, tj, crf_bc<F>(-1.0f));
+    const F nh = crf_fma(n, tj, nD);
+    const F nl = crf_fma(n, tj, crf_fma(nh, crf_bc<F>(-1.0f), nD));
 #pragma unroll
-        for (int i = 0; i < crf_lanes<F>::n; ++i) {
-            int j = crf_bits(crf_get(big, i)) - 0x4b400000;
-            j = j < 0 ? 0 : (j > 461 ? 461 : j);  // (in range for a <= 0.9; the other lanes are not used)
-            const float2 A = crf_ldg(lg_crf_atanh_tab + j);
-            crf_set(Ah, i, A.x);
-            crf_set(Al, i, A.y);
-        }
-        const F nh = crf_sub(a, tj);  // exact
-        const F qh = crf_mul(a, tj);
-        const F ql = crf_fma(a, tj, crf_neg(qh));
-        const F dh = crf_sub(one, qh);  // 1 >= qh: fast two-sum
-        const F dl = crf_sub(crf_sub(crf_sub(one, dh), qh), ql);
-#pragma unroll
-        for (int i = 0; i < crf_lanes<F>::n; ++i) crf_set(rd, i, crf_rcp(crf_get(dh, i)));  // dh in [0.19, 1]
-        const F d0 = crf_mul(nh, rd);
-        const F res = crf_fma(crf_neg(d0), dl, crf_fma(crf_neg(d0), dh, nh));
-        const F d1 = crf_mul(res, rd);
-        const F s = crf_mul(d0, d0);
-        const F P = crf_fma(s, crf_bc<F>(0x1.99999ap-3f), crf_bc<F>(0x1.555556p-2f));
-        const F cub = crf_mul(crf_mul(s, d0), P);
-        hs = crf_add(Ah, d0);  // |atanh t_j| >= |delta| or t_j = 0: fast two-sum
-        const F e1 = crf_sub(d0, crf_sub(hs, Ah));
-        ls = crf_add(crf_add(e1, Al), crf_add(d1, cub));
-    }
-    if (any_large) {
-        const F dh = crf_sub(one, a);
-        const F dl = crf_sub(crf_sub(one, dh), a);  // exact (1 >= a)
-        const F n = crf_add(a, a);
-        F rd;
-#pragma unroll
-        for (int i = 0; i < crf_lanes<F>::n; ++i) crf_set(rd, i, crf_rcp(crf_get(dh, i)));  // dh >= 2^-24
-        const F w0 = crf_mul(n, rd);
-        const F res = crf_fma(crf_neg(w0), dl, crf_fma(crf_neg(w0), dh, n));
-        const F w1 = crf_mul(res, rd);
-        // 1 + w0 (two-sum: w0 may exceed 1), + w1
-        const F uh = crf_add(one, w0);
-        const F bb = crf_sub(uh, one);
-        const F ul = crf_add(crf_add(crf_sub(one, crf_sub(uh, bb)), crf_sub(w0, bb)), w1);
-        crf_log_dw<F, true>(uh, ul, hl, ll);
-        hl = crf_mul(hl, crf_bc<F>(0.5f));
-        ll = crf_mul(ll, crf_bc<F>(0.5f));
-    }
-    F hi, lo;
-#pragma unroll
-    for (int i = 0; i < crf_lanes<F>::n; ++i) {
-        crf_set(hi, i, tab[i] ? crf_get(hs, i) : crf_get(hl, i));
-        crf_set(lo, i, tab[i] ? crf_get(ls, i) : crf_get(ll, i));
-    }
+    for (int i = 0; i < crf_lanes<F>::n; ++i) crf_set(rd, i, crf_rcp(-crf_get(nh, i)));
+    const F d = crf_mulx(n, rd);
+    const F d1 = crf_mulx(crf_fma(d, nl, crf_fma(d, nh, n)), rd);
+    const F c = crf_fma(crf_mulx(crf_mulx(d, d), d), crf_bc<F>(0x1.555556p-2f), d1);
+    const F s1 = crf_add(Ah, d);
+    const F ne = crf_fma(d, crf_bc<F>(-1.0f), crf_fma(Ah, crf_bc<F>(-1.0f), s1));
+    const F lo = crf_add(crf_fma(ne, crf_bc<F>(-1.0f), c), Al);
     F z1, z2;
-    crf_ziv(hi, lo, z1, z2);
-    // |v| < 1 with the rounding decided; |v| >= 1 and NaN v in double.  The
-    // sign of v on |result| (v = +-0 gives +-0).
-    bool ok2[2];
+    crf_quick_ziv(s1, lo, z1, z2);
     F out;
+    bool ok[2];
 #pragma unroll
     for (int i = 0; i < crf_lanes<F>::n; ++i) {
-        const float vi = crf_get(v, i);
-        ok2[i] = crf_fabsf(vi) < 1.0f && crf_get(z1, i) == crf_get(z2, i);
-        crf_set(out, i, crf_copysignf(crf_get(z1, i), vi));
+        ok[i] = crf_get(a, i) <= 0.9f && crf_get(z1, i) == crf_get(z2, i);
+        crf_set(out, i, crf_copysignf(crf_get(z1, i), crf_get(v, i)));
     }
-    if (crf_all<F>(ok2)) return out;
+    if (!crf_all<F>(ok)) {
 #pragma unroll
-    for (int i = 0; i < crf_lanes<F>::n; ++i)
-        if (!ok2[i]) crf_set(out, i, crf_slow_atanh(crf_get(v, i)));
+        for (int i = 0; i < crf_lanes<F>::n; ++i)
+            if (!ok[i]) crf_set(out, i, crf_rest_atanh(crf_get(v, i)));
+    }
     return out;
 }
 
@@ -730,7 +891,7 @@ LG_CRF_DEV void lg_crf_sincos(float x, float* sp, float* cp)
     const int j = crf_bits(bj) - 0x4b400000;  // |j| <= 201
     const float a = crf_mul(crf_sub(bj, S), 0x1p-8f);
     const float s0 = crf_sub(rh, a);  // exact
-    const float4 T = crf_ldg(lg_crf_sc_tab + (j + 201));
+    const float4 T = crf_tab4(lg_crf_sc_tab, (j + 201));
     const float sah = T.x, sal = T.y, cah = T.z, cal = T.w;
     // sin s = s0 + Sl; cos s - 1 = Ch + Cl
     const float s2 = crf_mul(s0, s0);
@@ -787,7 +948,7 @@ LG_CRF_DEV float lg_crf_pow(float x, float y)
     const bool xin = x >= 0x1p-126f && x <= 0x1.fffffep127f;
     const float xr = xin ? x : 1.0f;
     float lh, ll;
-    crf_log_dw<float, false>(xr, xr, lh, ll);
+    crf_log_dw<false>(xr, xr, lh, ll);
     const float th = crf_mul(y, lh);
     const float tl = crf_fma(y, ll, crf_fma(y, lh, -th));
     const bool tin = th >= -87.0f && th <= 88.0f;  // (false for NaN)
@@ -800,12 +961,12 @@ LG_CRF_DEV float lg_crf_pow(float x, float y)
     crf_two_sum(r0, tlo, rh, e);
     const float rl = crf_fma(-kf, LG_CRF_EXP_LLO, e);
     float yh, yl;
-    int m[2];
+    int m;
     crf_exp_tail(big, rh, rl, yh, yl, m);
     const float mrel = crf_fma(crf_fabsf(t), 0x1p-41f, LG_CRF_ZIV);
     const float mg = crf_mul(crf_fabsf(yh), mrel);
     const float z1 = crf_add(yh, crf_add(yl, mg)), z2 = crf_add(yh, crf_sub(yl, mg));
-    if (xin && tin && z1 == z2) return crf_from_bits(crf_add_exp(crf_bits(z1), m[0]));
+    if (xin && tin && z1 == z2) return crf_from_bits(crf_add_exp(crf_bits(z1), m));
     return crf_slow_pow(x, y);
 }
 

@@ -3,15 +3,20 @@ correctly rounded single-precision functions in lg_crfloat.cuh.
 
 Every value is computed with mpmath at 60 significant digits and rounded to
 float (round to nearest even) once; a "double-word" pair (hi, lo) holds
-hi = RN(v) and lo = RN(v - hi).
+hi = RN(v) and lo = RN(v - hi).  The tables are written as 64-bit words, two
+floats each: NVRTC reads them with every model it compiles, and one integer
+literal takes it a third of the time of a braced pair of float literals.
 
-  exp   T_j = 2^(j/64), j = 0..63, as (hi, lo)                (Tang 1989)
+  exp   T_j = 2^(j/64), j = 0..63, as (hi, lo)                (Tang 1989);
+        for the quick phase 2^(j/1024), j = 0..1023, as (hi, lo + D) with D
+        the half-width of its rounding interval
   log   for the 1024 intervals of the mantissa m in [0.75, 1.5) (512 of
         width 2^-11 below 1, 512 of width 2^-10 above): c_j = RN(1 / centre)
         (c = 1 for the two intervals next to 1) and -ln(c_j) as (hi, lo)
-        (Tang 1990)
+        (Tang 1990); for the quick phase -ln(c) of every c of 11 significant
+        bits from 1/2 - 2^-12 to 1, as (hi, lo) with hi a multiple of 2^-17
   atan  atan(j/512), j = 0..512, as (hi, lo)
-  atanh atanh(j/512), j = 0..461, as (hi, lo)
+  atanh atanh(j/512), j = 0..461, as (hi, lo) (padded to 512 entries)
   sin/cos  sin(j/256) and cos(j/256), j = -201..201, as (hi, lo) pairs
 
 Run:  python lensed_gb300/device/make_crf_tables.py
@@ -55,6 +60,12 @@ def lit(f: float) -> str:
     return f"{mant}p{exp}f"
 
 
+def word(*fs) -> str:
+    """Two (four) floats as one (two) 64-bit words, the first in the low half."""
+    b = [struct.unpack("I", struct.pack("f", f))[0] for f in fs]
+    return ", ".join(f"0x{b[i + 1]:08x}{b[i]:08x}u" for i in range(0, len(b), 2))
+
+
 def main():
     out = ["// generated by lensed_gb300/device/make_crf_tables.py -- do not edit",
            "// Tables of the correctly rounded single-precision functions (lg_crfloat.cuh).", ""]
@@ -62,8 +73,25 @@ def main():
     rows = []
     for j in range(64):
         hi, lo = split(mp.power(2, mp.mpf(j) / 64))
-        rows.append(f"{{{lit(hi)}, {lit(lo)}}}")
-    out.append("LG_CRF_TABLE(float2, lg_crf_exp_tab, 64) = {\n    " + ",\n    ".join(rows) + "};")
+        rows.append(word(hi, lo))
+    out.append("LG_CRF_TABLE(lg_crf_exp_tab, 64) = {\n    " + ",\n    ".join(rows) + "};")
+    # exp, quick phase: 2^(j/1024) as (hi, lo + D)
+    D = mp.mpf(float.fromhex("0x1.ap-35"))
+    rows = []
+    for j in range(1024):
+        v = mp.power(2, mp.mpf(j) / 1024)
+        hi = rn(v)
+        rows.append(word(hi, rn(v - mp.mpf(hi) + D)))
+    out.append("LG_CRF_TABLE(lg_crf_qexp_tab, 1024) = {\n    " + ",\n    ".join(rows) + "};")
+    # log, quick phase: -ln(c), c = float with bit pattern 0x3effe000 + j 2^13
+    rows = []
+    for j in range(1026):
+        c = struct.unpack("f", struct.pack("I", 0x3EFFE000 + (j << 13)))[0]
+        v = -mp.log(mp.mpf(c))
+        hi = mp.floor(v * 2 ** 17 + mp.mpf(0.5)) / 2 ** 17
+        assert mp.mpf(rn(hi)) == hi
+        rows.append(word(rn(hi), rn(v - hi)))
+    out.append("LG_CRF_TABLE(lg_crf_qlog_tab, 1026) = {\n    " + ",\n    ".join(rows) + "};")
     # log: (c, -ln c hi, -ln c lo, 0)
     rows = []
     for j in range(1024):
@@ -73,33 +101,38 @@ def main():
             m0, w = 1 + (j - 512) * mp.mpf(2) ** -10, mp.mpf(2) ** -10
         c = 1.0 if j in (511, 512) else rn(1 / (m0 + w / 2))
         hi, lo = split(-mp.log(mp.mpf(c)))
-        rows.append(f"{{{lit(c)}, {lit(hi)}, {lit(lo)}, 0.0f}}")
-    out.append("LG_CRF_TABLE(float4, lg_crf_log_tab, 1024) = {\n    " + ",\n    ".join(rows) + "};")
+        rows.append(word(c, hi, lo, 0.0))
+    out.append("LG_CRF_TABLE(lg_crf_log_tab, 2 * 1024) = {\n    " + ",\n    ".join(rows) + "};")
     # atan(j/512)
     rows = []
     for j in range(513):
         hi, lo = split(mp.atan(mp.mpf(j) / 512))
-        rows.append(f"{{{lit(hi)}, {lit(lo)}}}")
-    out.append("LG_CRF_TABLE(float2, lg_crf_atan_tab, 513) = {\n    " + ",\n    ".join(rows) + "};")
+        rows.append(word(hi, lo))
+    out.append("LG_CRF_TABLE(lg_crf_atan_tab, 513) = {\n    " + ",\n    ".join(rows) + "};")
     # atanh(j/512), j = 0..461, as (hi, lo)
     rows = []
     for j in range(462):
         hi, lo = split(mp.atanh(mp.mpf(j) / 512))
-        rows.append(f"{{{lit(hi)}, {lit(lo)}}}")
-    out.append("LG_CRF_TABLE(float2, lg_crf_atanh_tab, 462) = {\n    " + ",\n    ".join(rows) + "};")
+        rows.append(word(hi, lo))
+    out.append("LG_CRF_TABLE(lg_crf_atanh_tab, 512) = {\n    " + ",\n    ".join(rows) + "};")
     # sin / cos(j/256), j = -201..201, as (sin hi, sin lo, cos hi, cos lo)
     rows = []
     for j in range(-201, 202):
         a = mp.mpf(j) / 256
         sh, sl = split(mp.sin(a))
         ch, cl = split(mp.cos(a))
-        rows.append(f"{{{lit(sh)}, {lit(sl)}, {lit(ch)}, {lit(cl)}}}")
-    out.append("LG_CRF_TABLE(float4, lg_crf_sc_tab, 403) = {\n    " + ",\n    ".join(rows) + "};")
+        rows.append(word(sh, sl, ch, cl))
+    out.append("LG_CRF_TABLE(lg_crf_sc_tab, 2 * 403) = {\n    " + ",\n    ".join(rows) + "};")
     # split constants
     consts = {}
     l64 = mp.log(2) / 64
     consts["LG_CRF_EXP_INVL"] = rn(64 / mp.log(2))
     consts["LG_CRF_EXP_LHI"], consts["LG_CRF_EXP_LLO"] = split(l64)
+    # quick phases: ln2/1024 = L_hi + L_lo; ln2 2^-23 = (multiple of 2^-40) + rest
+    consts["LG_CRF_QEXP_INVL"] = rn(1024 / mp.log(2))
+    consts["LG_CRF_QEXP_LHI"], consts["LG_CRF_QEXP_LLO"] = split(mp.log(2) / 1024)
+    h = mp.floor(mp.log(2) * 2 ** 17 + mp.mpf(0.5)) / 2 ** 17
+    consts["LG_CRF_QLN2_HI"], consts["LG_CRF_QLN2_LO"] = rn(h * mp.mpf(2) ** -23), rn((mp.log(2) - h) * mp.mpf(2) ** -23)
     consts["LG_CRF_LN2_HI"], consts["LG_CRF_LN2_LO"] = split(mp.log(2))
     consts["LG_CRF_PIO2_HI"], consts["LG_CRF_PIO2_LO"] = split(mp.pi / 2)
     # sin / cos argument reduction: 2/pi, and pi/2 = P1 + P2 + P3 with P1
