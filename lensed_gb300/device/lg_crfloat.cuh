@@ -75,6 +75,7 @@ LG_CRF_DEV float crf_from_bits(int i)
 #define LG_CRF_HOST_RCP(a) (1.0f / (a))
 #endif
 LG_CRF_DEV float crf_rcp(float a) { return LG_CRF_HOST_RCP(a); }
+LG_CRF_DEV float crf_rsqrt(float a) { return LG_CRF_HOST_RCP(std::sqrt(a)); }
 // (a test build may count the lanes that take the double path)
 #ifndef LG_CRF_SLOW_COUNT
 #define LG_CRF_SLOW_COUNT()
@@ -112,9 +113,13 @@ LG_CRF_DEV float crf_add(float a, float b) { return __fadd_rn(a, b); }
 LG_CRF_DEV float crf_sub(float a, float b) { return __fsub_rn(a, b); }
 LG_CRF_DEV float crf_mul(float a, float b) { return __fmul_rn(a, b); }
 LG_CRF_DEV float crf_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-// paired operations on f32x2: add and fma.  (With CUDA 13.0 the assembler
-// fused an f32x2 multiply into a following f32x2 add; see crf_mulx for the
-// products of the quick phases.)
+// paired operations on f32x2.  With CUDA 13.0 the assembler fused an f32x2
+// multiply into a following f32x2 add (also without contraction), so a
+// product that must be rounded first is an fma with -0 (the same value for
+// every operand), read from memory so that the assembler cannot see it.
+// Negated and absolute operands are free (instruction modifiers).
+__constant__ float2 crf_negzero = {-0.0f, -0.0f};
+LG_CRF_DEV float2 crf_mul(float2 a, float2 b) { return __ffma2_rn(a, b, crf_negzero); }
 LG_CRF_DEV float2 crf_add(float2 a, float2 b) { return __fadd2_rn(a, b); }
 LG_CRF_DEV float2 crf_sub(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
 LG_CRF_DEV float2 crf_fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
@@ -126,6 +131,13 @@ LG_CRF_DEV float crf_rcp(float a)
 {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
+// PTX rsqrt.approx (within about 2 ulp)
+LG_CRF_DEV float crf_rsqrt(float a)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
     return r;
 }
 // Integer fields of the arguments' bit patterns, in inline PTX: with CUDA
@@ -244,6 +256,42 @@ LG_CRF_DEV float2 crf_abs(float2 a)
 // (the library embeds the tables here for NVRTC, which has no include path)
 #ifndef LG_CRF_TABLES_INLINE
 #include "lg_crf_tables.cuh"
+#endif
+
+// Entry of a quick-phase table: base (LG_CRF_Q_*) plus a byte offset.  With
+// LG_CRF_SMEM the tables (24.6 KB) are read from a copy in shared memory that
+// the kernel fills with crf_load_tables first: a lookup is then two or three
+// instructions (32-bit offsets, the table's address an immediate) instead of
+// the five of a global load with its 64-bit address, and the table reads are
+// a fifth of the quick phases' instructions.
+#if defined(LG_CRF_HOST)
+LG_CRF_DEV float2 crf_qtab(int base, unsigned off)
+{
+    float2 v;
+    std::memcpy(&v, lg_crf_q_tab + base + off / 8, 8);
+    return v;
+}
+#elif defined(LG_CRF_SMEM)
+__shared__ __align__(16) unsigned long long lg_crf_s[LG_CRF_Q_ENTRIES];
+LG_CRF_DEV float2 crf_qtab(int base, unsigned off)
+{
+    return *reinterpret_cast<const float2*>(reinterpret_cast<const char*>(lg_crf_s) + 8 * base + off);
+}
+// every thread of the block (NT threads) calls it, before any lookup
+template <int NT>
+LG_CRF_DEV void crf_load_tables(int tid)
+{
+    const float4* src = reinterpret_cast<const float4*>(lg_crf_q_tab);
+    float4* dst = reinterpret_cast<float4*>(lg_crf_s);
+#pragma unroll 4
+    for (int i = tid; i < LG_CRF_Q_ENTRIES / 2; i += NT) dst[i] = __ldg(src + i);
+    __syncthreads();
+}
+#else
+LG_CRF_DEV float2 crf_qtab(int base, unsigned off)
+{
+    return __ldg(reinterpret_cast<const float2*>(reinterpret_cast<const char*>(lg_crf_q_tab) + 8 * base + off));
+}
 #endif
 
 // Relative half-width of Ziv's interval: the double-word results of the
@@ -449,7 +497,7 @@ LG_CRF_DEV void crf_atan_core(float th, float tl, float& s1, float& lo)
     const float tj = crf_mul(crf_sub(big, S), 0x1p-9f);
     int j = crf_bits(big) - 0x4b400000;
     j = j < 0 ? 0 : (j > 512 ? 512 : j);  // (in range for every finite t in [0, 1])
-    const float2 A = crf_tab2(lg_crf_atan_tab, j);
+    const float2 A = crf_tab2(lg_crf_q_tab + LG_CRF_Q_ATAN, j);
     const float Ah = A.x, Al = A.y;
     const float nh = crf_sub(th, tj);  // exact
     const float qh = crf_mul(th, tj);
@@ -515,7 +563,7 @@ LG_CRF_DEV float crf_full_atanh(float v)
         const float S = 0x1.8p23f;
         const float big = crf_fma(a, 512.0f, S);
         const float tj = crf_mul(crf_sub(big, S), 0x1p-9f);
-        const float2 A = crf_tab2(lg_crf_atanh_tab, crf_bits(big) - 0x4b400000);
+        const float2 A = crf_tab2(lg_crf_q_tab + LG_CRF_Q_ATANH, crf_bits(big) - 0x4b400000);
         const float Ah = A.x, Al = A.y;
         const float nh = crf_sub(a, tj);  // exact
         const float qh = crf_mul(a, tj);
@@ -625,7 +673,7 @@ LG_CRF_DEV F lg_crf_exp(F x)
     F th, tl;
 #pragma unroll
     for (int i = 0; i < crf_lanes<F>::n; ++i) {
-        const float2 T = crf_tab2(lg_crf_qexp_tab, (crf_bits(crf_get(big, i)) & 1023));
+        const float2 T = crf_qtab(LG_CRF_Q_EXP, (unsigned)(crf_bits(crf_get(big, i)) & 1023) * 8u);
         crf_set(th, i, T.x);
         crf_set(tl, i, T.y);
     }
@@ -655,8 +703,9 @@ LG_CRF_DEV F lg_crf_exp(F x)
 // first sum is exact.  Absolute error: the sum with r (2^-34 at most, the
 // rest of it reaching 2^-11), e ln2_lo + Ll (2^-36), r^4/4 (2^-42); D =
 // 1.375 2^-34.  Results near 0 are left to the full phase.
+// Out: s1, r and t with ln x = s1 + (r + t).
 template <class F>
-LG_CRF_DEV F lg_crf_log(F x)
+LG_CRF_DEV void crf_quick_log(F x, F& s1, F& r, F& t)
 {
     F m, c, Lh, Ll, ef;
 #pragma unroll
@@ -664,19 +713,25 @@ LG_CRF_DEV F lg_crf_log(F x)
         int mb, te;
         crf_qlog_fields(crf_bits(crf_get(x, i)), mb, te);
         const int cb = crf_bits(crf_rcp(crf_from_bits(mb))) & (int)0xffffe000;
-        const float2 T = crf_tab2(lg_crf_qlog_tab, (int)((unsigned)cb >> 13) - (0x3effe000 >> 13));
+        const float2 T = crf_qtab(LG_CRF_Q_LOG, ((unsigned)cb >> 10) - (0x3effe000u >> 10));
         crf_set(m, i, crf_from_bits(mb));
         crf_set(c, i, crf_from_bits(cb));
         crf_set(Lh, i, T.x);
         crf_set(Ll, i, T.y);
         crf_set(ef, i, (float)te);  // exact
     }
-    const F r = crf_fma(m, c, crf_bc<F>(-1.0f));
+    r = crf_fma(m, c, crf_bc<F>(-1.0f));
     const F e = crf_add(ef, crf_bc<F>(-127.0f * 0x1p23f));
-    const F s1 = crf_fma(e, crf_bc<F>(LG_CRF_QLN2_HI), Lh);
+    s1 = crf_fma(e, crf_bc<F>(LG_CRF_QLN2_HI), Lh);
     const F lo = crf_fma(e, crf_bc<F>(LG_CRF_QLN2_LO), Ll);
     const F w = crf_fma(r, crf_bc<F>(0x1.555556p-2f), crf_bc<F>(-0.5f));
-    const F t = crf_fma(crf_mulx(r, r), w, lo);
+    t = crf_fma(crf_mulx(r, r), w, lo);
+}
+template <class F>
+LG_CRF_DEV F lg_crf_log(F x)
+{
+    F s1, r, t;
+    crf_quick_log(x, s1, r, t);
     const F z1 = crf_add(s1, crf_add(r, crf_add(t, crf_bc<F>(0x1.6p-34f))));
     const F z2 = crf_add(s1, crf_add(r, crf_add(t, crf_bc<F>(-0x1.6p-34f))));
     F out = z1;
@@ -700,7 +755,8 @@ LG_CRF_DEV void crf_quick_ziv(F hi, F lo, F& z1, F& z2)
     z2 = crf_add(hi, crf_fma(hi, crf_bc<F>(-0x1p-38f), lo));
 }
 
-// atan t for t in [0, 1]: with t_j = j/512 nearest t, n = t - t_j and d = n /
+// atan t for t in [0, 1] (callers keep every t, NaN included, in that range:
+// it indexes the table): with t_j = j/512 nearest t, n = t - t_j and d = n /
 // (1 + t_j^2) (the denominator exact), atan t = atan t_j + d - t_j d^2 + (t_j^2
 // - 1/3) d^3 + O(d^4 t_j) (Taylor's series in d; |d| <= 2^-10, the omitted
 // term 2^-40 of the result).  d as a double word from the reciprocal estimate
@@ -714,7 +770,7 @@ LG_CRF_DEV void crf_quick_atan(F t, F tl, F& s1, F& lo)
     F Ah, Al, nr;
 #pragma unroll
     for (int i = 0; i < crf_lanes<F>::n; ++i) {
-        const float2 A = crf_tab2(lg_crf_atan_tab, (crf_bits(crf_get(big, i)) - 0x46c00000));
+        const float2 A = crf_qtab(LG_CRF_Q_ATAN, (unsigned)(crf_bits(crf_get(big, i)) - 0x46c00000) * 8u);
         crf_set(Ah, i, A.x);
         crf_set(Al, i, A.y);
     }
@@ -727,7 +783,9 @@ LG_CRF_DEV void crf_quick_atan(F t, F tl, F& s1, F& lo)
     if (DW) res = crf_add(res, tl);
     F nd1 = crf_mulx(res, nr);
     if (DW) nd1 = crf_fma(crf_add(nd1, nd1), crf_mulx(tj, nd), nd1);  // the square's cross term with tl
-    const F P = crf_fma(crf_add(s, crf_bc<F>(-0x1.555556p+0f)), nd, tj);
+    F K = crf_add(s, crf_bc<F>(-0x1.555556p+0f));
+    if (DW) K = crf_fma(crf_mulx(tj, crf_add(s, crf_bc<F>(-2.0f))), nd, K);  // the fourth power's term
+    const F P = crf_fma(K, nd, tj);
     const F nc = crf_fma(crf_mulx(nd, nd), P, nd1);
     s1 = crf_fma(nd, crf_bc<F>(-1.0f), Ah);
     const F ne = crf_add(nd, crf_fma(Ah, crf_bc<F>(-1.0f), s1));
@@ -809,7 +867,7 @@ LG_CRF_DEV F lg_crf_atanh(F v)
 #pragma unroll
     for (int i = 0; i < crf_lanes<F>::n; ++i) {
         // (the mask keeps arguments outside the range inside the table)
-        const float2 A = crf_tab2(lg_crf_atanh_tab, (crf_bits(crf_get(big, i)) & 511));
+        const float2 A = crf_qtab(LG_CRF_Q_ATANH, (unsigned)(crf_bits(crf_get(big, i)) & 511) * 8u);
         crf_set(Ah, i, A.x);
         crf_set(Al, i, A.y);
     }
@@ -1013,4 +1071,170 @@ LG_CRF_DEV float lg_crf_atan2(float y, float x)
     float z;
     if (in && crf_ziv1(hi, lo, 0.0f, z)) return crf_copysignf(z, y);
     return crf_slow_atan2(y, x);
+}
+
+// ------------------------------------------- quick phases of the EPL lens --
+// x^y for one exponent: ln x = s1 + a from the quick log (a its float part,
+// absolute error 1.375 2^-34 with its rounding), t = y ln x as a double word
+// (y s1 exactly, y a added, a two-sum; error |y| 1.875 2^-34), e^t as in
+// lg_crf_exp with the low part added to the reduction's.  The interval of
+// the exp widened by twice that error.  Positive normal x with |t| <= 86;
+// the rest, and undecided roundings, in the full phase.
+LG_CRF_COLD float crf_rest_pow(float x, float y) { LG_CRF_REST_COUNT(); return lg_crf_pow(x, y); }
+template <class F>
+LG_CRF_DEV F lg_crf_pow1(F x, float y)
+{
+    F s1, r, t;
+    crf_quick_log(x, s1, r, t);
+    const F a = crf_add(r, t);
+    const F Y = crf_bc<F>(y);
+    const F ph = crf_mul(Y, s1);
+    const F pl = crf_fma(Y, a, crf_fma(Y, s1, crf_neg(ph)));
+    const F T = crf_add(ph, pl);  // two-sum
+    const F bb = crf_sub(T, ph);
+    const F Tl = crf_add(crf_sub(ph, crf_sub(T, bb)), crf_sub(pl, bb));
+    const F big = crf_fma(T, crf_bc<F>(LG_CRF_QEXP_INVL), crf_bc<F>(0x1.8p23f));
+    const F kf = crf_add(big, crf_bc<F>(-0x1.8p23f));
+    const F rh = crf_fma(kf, crf_bc<F>(-LG_CRF_QEXP_LHI), T);
+    const F rl = crf_fma(kf, crf_bc<F>(-LG_CRF_QEXP_LLO), Tl);
+    const F sm = crf_fma(rh, crf_fma(rh, crf_bc<F>(0.5f), rl), rl);
+    F th, tl;
+#pragma unroll
+    for (int i = 0; i < crf_lanes<F>::n; ++i) {
+        const float2 E = crf_qtab(LG_CRF_Q_EXP, (unsigned)(crf_bits(crf_get(big, i)) & 1023) * 8u);
+        crf_set(th, i, E.x);
+        crf_set(tl, i, E.y);
+    }
+    const float wide = crf_mul(crf_fabsf(y), 0x1p-32f);
+    const F w0 = crf_fma(th, sm, crf_fma(tl, rh, tl));
+    const F w1 = crf_add(w0, crf_bc<F>(wide));
+    const F w2 = crf_sub(w0, crf_bc<F>(crf_add(wide, 0x1.ap-34f)));
+    const F z1 = crf_add(th, crf_fma(th, rh, w1));
+    const F z2 = crf_add(th, crf_fma(th, rh, w2));
+    F out;
+    bool ok[2];
+#pragma unroll
+    for (int i = 0; i < crf_lanes<F>::n; ++i) {
+        ok[i] = (unsigned)crf_bits(crf_get(x, i)) - 0x00800000u < 0x7f000000u && crf_fabsf(crf_get(T, i)) <= 86.0f &&
+                crf_get(z1, i) == crf_get(z2, i);
+        crf_set(out, i, crf_from_bits(crf_qexp_scale(crf_bits(crf_get(z1, i)), crf_bits(crf_get(big, i)))));
+    }
+    if (!crf_all<F>(ok)) {
+#pragma unroll
+        for (int i = 0; i < crf_lanes<F>::n; ++i)
+            if (!ok[i]) crf_set(out, i, crf_rest_pow(crf_get(x, i), y));
+    }
+    return out;
+}
+
+// The EPL lens's polar frame of a point (X, Y): r = sqrt(X^2 + Y^2) with
+// every operation rounded, phi = atan2(Y, X) rounded, and the sine and
+// cosine of that float phi and of 2 phi, each correctly rounded, in one
+// computation instead of an atan2 and two sincos:
+//  * H = X^2 + Y^2 as a double word (exact products; its high part is the
+//    rounded sum r is the root of), 1/sqrt(H) = y0 + y1 from the reciprocal
+//    square root estimate and one Newton step (error 2^-44), so cos and sin
+//    of the exact angle are X and Y times it;
+//  * the exact angle from the atan of min/max as in lg_crf_atan, then phi =
+//    its rounding, and rem = angle - phi;
+//  * sin phi = sin(angle) - rem cos(angle), cos phi likewise (rem^2/2 is
+//    below 2^-45), sin 2phi = 2 sin phi cos phi, cos 2phi = +-(1 - 2 m^2) with
+//    m the smaller of the two.
+// The rounding tests' margins are twice the largest errors measured with
+// reciprocal estimates 2^-22 off: sin phi and sin phi cos phi 2^-38.5 |phi|
+// and 2^-40, cos phi 2^-40, cos 2phi 2^-39.  ok[i]: every rounding of lane i decided; its range
+// excludes axes and extreme sizes (min/max < 2^-20, H outside [2^-60,
+// 2^60]), which the caller sends through the one-value functions.
+template <class F>
+LG_CRF_DEV void crf_quick_polar(F X, F Y, F& r, F& c, F& s, F& c2, F& s2, bool (&ok)[2])
+{
+    F den, num, y0, rd;
+    bool swap[2];
+#pragma unroll
+    for (int i = 0; i < crf_lanes<F>::n; ++i) {
+        const float ax = crf_fabsf(crf_get(X, i)), ay = crf_fabsf(crf_get(Y, i));
+        swap[i] = ay > ax;
+        crf_set(den, i, swap[i] ? ay : ax);
+        crf_set(num, i, swap[i] ? ax : ay);
+    }
+    const F A = crf_mul(den, den), B = crf_mul(num, num);
+    const F h = crf_add(A, B);
+    const F hl = crf_add(crf_sub(B, crf_sub(h, A)), crf_add(crf_fma(den, den, crf_neg(A)), crf_fma(num, num, crf_neg(B))));
+#pragma unroll
+    for (int i = 0; i < crf_lanes<F>::n; ++i) {
+        crf_set(y0, i, crf_rsqrt(crf_get(h, i)));
+        crf_set(rd, i, crf_rcp(crf_get(den, i)));
+    }
+    // r
+    const F g = crf_mul(h, y0);
+    const F hy = crf_mulx(y0, crf_bc<F>(0.5f));
+    const F g1 = crf_mulx(crf_fma(crf_neg(g), g, h), hy);
+    r = crf_add(g, crf_fma(g, crf_bc<F>(0x1p-40f), g1));
+    const F r2 = crf_add(g, crf_fma(g, crf_bc<F>(-0x1p-40f), g1));
+    // 1/sqrt(H) = y0 + y1; cos, sin of the exact angle
+    const F pe = crf_fma(hl, y0, crf_fma(h, y0, crf_neg(g)));
+    const F y1 = crf_mulx(hy, crf_fma(crf_neg(pe), y0, crf_fma(crf_neg(g), y0, crf_bc<F>(1.0f))));
+    const F ch = crf_mul(X, y0), sh = crf_mul(Y, y0);
+    F cl = crf_fma(X, y1, crf_fma(X, y0, crf_neg(ch)));
+    F sl = crf_fma(Y, y1, crf_fma(Y, y0, crf_neg(sh)));
+    // the angle in [0, pi]: B + sg atan(num/den)
+    F q0 = crf_mul(num, rd);
+#pragma unroll
+    for (int i = 0; i < crf_lanes<F>::n; ++i)  // NaN and infinite quotients (left undecided) stay inside the table
+        crf_set(q0, i, crf_get(q0, i) <= 1.0f ? crf_get(q0, i) : 1.0f);
+    const F q1 = crf_mulx(crf_fma(crf_neg(q0), den, num), rd);
+    F ah, al, Bh, Bl, sg;
+    crf_quick_atan<F, true>(q0, q1, ah, al);
+#pragma unroll
+    for (int i = 0; i < crf_lanes<F>::n; ++i) {
+        const bool neg = crf_get(X, i) < 0.0f;
+        crf_set(sg, i, swap[i] != neg ? -1.0f : 1.0f);
+        crf_set(Bh, i, swap[i] ? LG_CRF_PIO2_HI : (neg ? 2.0f * LG_CRF_PIO2_HI : 0.0f));
+        crf_set(Bl, i, swap[i] ? LG_CRF_PIO2_LO : (neg ? 2.0f * LG_CRF_PIO2_LO : 0.0f));
+    }
+    const F zh = crf_fma(sg, ah, Bh);
+    const F zl = crf_fma(sg, al, crf_add(crf_fma(sg, ah, crf_sub(Bh, zh)), Bl));
+    F z1, z2;
+    crf_quick_ziv(zh, zl, z1, z2);
+    // rem = angle - phi, with the sign of Y; sin, cos of phi
+    F rem = crf_add(zl, crf_sub(zh, z1));
+#pragma unroll
+    for (int i = 0; i < crf_lanes<F>::n; ++i)
+        crf_set(rem, i, crf_from_bits(crf_bits(crf_get(rem, i)) ^ (crf_bits(crf_get(Y, i)) & (int)0x80000000)));
+    sl = crf_fma(crf_neg(rem), ch, sl);
+    cl = crf_fma(rem, sh, cl);
+    F ms = crf_mulx(z1, crf_bc<F>(0x1.6p-39f));
+#pragma unroll
+    for (int i = 0; i < crf_lanes<F>::n; ++i) crf_set(ms, i, crf_get(ms, i) < 0x1p-40f ? crf_get(ms, i) : 0x1p-40f);
+    const F mc = crf_bc<F>(0x1p-40f), mk = crf_bc<F>(0x1p-39f);
+    s = crf_add(sh, crf_add(sl, ms));
+    const F sb = crf_add(sh, crf_sub(sl, ms));
+    c = crf_add(ch, crf_add(cl, mc));
+    const F cb = crf_add(ch, crf_sub(cl, mc));
+    // sin 2phi
+    const F ph = crf_mul(sh, ch);
+    const F pl = crf_fma(sh, cl, crf_fma(sl, ch, crf_fma(sh, ch, crf_neg(ph))));
+    s2 = crf_add(ph, crf_add(pl, ms));
+    const F s2b = crf_add(ph, crf_sub(pl, ms));
+    // cos 2phi
+    F mh, ml;
+#pragma unroll
+    for (int i = 0; i < crf_lanes<F>::n; ++i) {
+        crf_set(mh, i, swap[i] ? crf_get(ch, i) : crf_get(sh, i));
+        crf_set(ml, i, swap[i] ? crf_get(cl, i) : crf_get(sl, i));
+    }
+    const F q = crf_mul(mh, mh);
+    const F qe = crf_fma(crf_mulx(mh, ml), crf_bc<F>(2.0f), crf_fma(mh, mh, crf_neg(q)));
+    const F k = crf_fma(q, crf_bc<F>(-2.0f), crf_bc<F>(1.0f));
+    const F ke = crf_fma(qe, crf_bc<F>(-2.0f), crf_fma(q, crf_bc<F>(-2.0f), crf_sub(crf_bc<F>(1.0f), k)));
+    const F k1 = crf_add(k, crf_add(ke, mk));
+    const F k2 = crf_add(k, crf_sub(ke, mk));
+#pragma unroll
+    for (int i = 0; i < crf_lanes<F>::n; ++i) {
+        crf_set(c2, i, swap[i] ? -crf_get(k1, i) : crf_get(k1, i));
+        ok[i] = crf_get(h, i) >= 0x1p-60f && crf_get(h, i) <= 0x1p60f && crf_get(q0, i) >= 0x1p-20f &&
+                crf_get(r, i) == crf_get(r2, i) && crf_get(z1, i) == crf_get(z2, i) && crf_get(s, i) == crf_get(sb, i) &&
+                crf_get(c, i) == crf_get(cb, i) && crf_get(s2, i) == crf_get(s2b, i) && crf_get(k1, i) == crf_get(k2, i);
+    }
+    s2 = crf_add(s2, s2);
 }

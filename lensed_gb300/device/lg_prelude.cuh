@@ -130,11 +130,14 @@ struct lg_pair {
 // product must be rounded before the sum that uses it; with CUDA 13.0 the
 // assembler fused an f32x2 multiply into the following f32x2 add (the
 // intrinsics and explicit-rounding PTX alike, also without contraction
-// enabled), while scalar round-to-nearest multiplies are never fused.  So
-// the exact modules multiply lane by lane (__fmul_rn) and keep the paired
-// add and fma; the fast modules use the paired intrinsics throughout.
+// enabled).  There a product is an fma with -0 (the same value for every
+// operand), read from memory so that the assembler cannot see it: half the
+// instructions of lane-by-lane multiplies, and scalar FP32 instructions
+// between f32x2 ones take the pipe as long as those (measured: an f32x2 fma
+// and a scalar add 4.2 cycles, two f32x2 4.3).
 #ifdef LG_EXACT
-LG_DEV float2 lg_mul2(float2 a, float2 b) { return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y)); }
+__constant__ float2 lg_negzero = {-0.0f, -0.0f};
+LG_DEV float2 lg_mul2(float2 a, float2 b) { return __ffma2_rn(a, b, lg_negzero); }
 #else
 LG_DEV float2 lg_mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 #endif

@@ -16,7 +16,7 @@ literal takes it a third of the time of a braced pair of float literals.
         (Tang 1990); for the quick phase -ln(c) of every c of 11 significant
         bits from 1/2 - 2^-12 to 1, as (hi, lo) with hi a multiple of 2^-17
   atan  atan(j/512), j = 0..512, as (hi, lo)
-  atanh atanh(j/512), j = 0..461, as (hi, lo) (padded to 512 entries)
+  atanh atanh(j/512), j = 0..461, as (hi, lo), padded to 512 entries
   sin/cos  sin(j/256) and cos(j/256), j = -201..201, as (hi, lo) pairs
 
 Run:  python lensed_gb300/device/make_crf_tables.py
@@ -75,23 +75,6 @@ def main():
         hi, lo = split(mp.power(2, mp.mpf(j) / 64))
         rows.append(word(hi, lo))
     out.append("LG_CRF_TABLE(lg_crf_exp_tab, 64) = {\n    " + ",\n    ".join(rows) + "};")
-    # exp, quick phase: 2^(j/1024) as (hi, lo + D)
-    D = mp.mpf(float.fromhex("0x1.ap-35"))
-    rows = []
-    for j in range(1024):
-        v = mp.power(2, mp.mpf(j) / 1024)
-        hi = rn(v)
-        rows.append(word(hi, rn(v - mp.mpf(hi) + D)))
-    out.append("LG_CRF_TABLE(lg_crf_qexp_tab, 1024) = {\n    " + ",\n    ".join(rows) + "};")
-    # log, quick phase: -ln(c), c = float with bit pattern 0x3effe000 + j 2^13
-    rows = []
-    for j in range(1026):
-        c = struct.unpack("f", struct.pack("I", 0x3EFFE000 + (j << 13)))[0]
-        v = -mp.log(mp.mpf(c))
-        hi = mp.floor(v * 2 ** 17 + mp.mpf(0.5)) / 2 ** 17
-        assert mp.mpf(rn(hi)) == hi
-        rows.append(word(rn(hi), rn(v - hi)))
-    out.append("LG_CRF_TABLE(lg_crf_qlog_tab, 1026) = {\n    " + ",\n    ".join(rows) + "};")
     # log: (c, -ln c hi, -ln c lo, 0)
     rows = []
     for j in range(1024):
@@ -103,18 +86,45 @@ def main():
         hi, lo = split(-mp.log(mp.mpf(c)))
         rows.append(word(c, hi, lo, 0.0))
     out.append("LG_CRF_TABLE(lg_crf_log_tab, 2 * 1024) = {\n    " + ",\n    ".join(rows) + "};")
+    # exp, quick phase: 2^(j/1024) as (hi, lo + D)
+    D = mp.mpf(float.fromhex("0x1.ap-35"))
+    rows = []
+    for j in range(1024):
+        v = mp.power(2, mp.mpf(j) / 1024)
+        hi = rn(v)
+        rows.append(word(hi, rn(v - mp.mpf(hi) + D)))
+    quick = {"EXP": rows}
+    # log, quick phase: -ln(c), c = float with bit pattern 0x3effe000 + j 2^13
+    rows = []
+    for j in range(1026):
+        c = struct.unpack("f", struct.pack("I", 0x3EFFE000 + (j << 13)))[0]
+        v = -mp.log(mp.mpf(c))
+        hi = mp.floor(v * 2 ** 17 + mp.mpf(0.5)) / 2 ** 17
+        assert mp.mpf(rn(hi)) == hi
+        rows.append(word(rn(hi), rn(v - hi)))
+    quick["LOG"] = rows
     # atan(j/512)
     rows = []
     for j in range(513):
         hi, lo = split(mp.atan(mp.mpf(j) / 512))
         rows.append(word(hi, lo))
-    out.append("LG_CRF_TABLE(lg_crf_atan_tab, 513) = {\n    " + ",\n    ".join(rows) + "};")
-    # atanh(j/512), j = 0..461, as (hi, lo)
+    quick["ATAN"] = rows
+    # atanh(j/512), j = 0..461, as (hi, lo), padded to 512 entries
     rows = []
     for j in range(462):
         hi, lo = split(mp.atanh(mp.mpf(j) / 512))
         rows.append(word(hi, lo))
-    out.append("LG_CRF_TABLE(lg_crf_atanh_tab, 512) = {\n    " + ",\n    ".join(rows) + "};")
+    rows += [word(0.0, 0.0)] * 50
+    quick["ATANH"] = rows
+    # the tables of the quick phases in one array, copied to shared memory as a
+    # whole; LG_CRF_Q_*: first entry of each
+    allrows = []
+    for name, r in quick.items():
+        out.append(f"#define LG_CRF_Q_{name} {len(allrows)}")
+        allrows += r
+    allrows += [word(0.0, 0.0)] * (len(allrows) % 2)
+    out.append(f"#define LG_CRF_Q_ENTRIES {len(allrows)}")
+    out.append(f"LG_CRF_TABLE(lg_crf_q_tab, {len(allrows)}) = {{\n    " + ",\n    ".join(allrows) + "};")
     # sin / cos(j/256), j = -201..201, as (sin hi, sin lo, cos hi, cos lo)
     rows = []
     for j in range(-201, 202):

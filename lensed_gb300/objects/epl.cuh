@@ -40,11 +40,31 @@ LG_DEV void lg_polar(float2 x, float* r, float* c, float* s, float* c2, float* s
     sincosf(2 * phi, s2, c2);
 }
 #if defined(LG_EXACT) && !defined(LG_HOST_SET)
-// the exact modules trace ray pairs with the one-ray calls, lane by lane
+// the exact modules' ray pairs: both rays in one computation, a ray it
+// leaves undecided with the one-ray calls (out of line)
+struct lg_polar_values {
+    float r, c, s, c2, s2;
+};
+static __device__ __noinline__ lg_polar_values lg_polar_rest(float2 x)
+{
+    lg_polar_values v;
+    lg_polar(x, &v.r, &v.c, &v.s, &v.c2, &v.s2);
+    return v;
+}
 LG_DEV void lg_polar(lg_pair2 x, lg_pair* r, lg_pair* c, lg_pair* s, lg_pair* c2, lg_pair* s2)
 {
-    lg_polar(lg_lane(x, 0), &r->v.x, &c->v.x, &s->v.x, &c2->v.x, &s2->v.x);
-    lg_polar(lg_lane(x, 1), &r->v.y, &c->v.y, &s->v.y, &c2->v.y, &s2->v.y);
+    bool ok[2];
+    crf_quick_polar(x.x.v, x.y.v, r->v, c->v, s->v, c2->v, s2->v, ok);
+    if (!(ok[0] && ok[1])) {
+        if (!ok[0]) {
+            const lg_polar_values v = lg_polar_rest(lg_lane(x, 0));
+            r->v.x = v.r; c->v.x = v.c; s->v.x = v.s; c2->v.x = v.c2; s2->v.x = v.s2;
+        }
+        if (!ok[1]) {
+            const lg_polar_values v = lg_polar_rest(lg_lane(x, 1));
+            r->v.y = v.r; c->v.y = v.c; s->v.y = v.s; c2->v.y = v.c2; s2->v.y = v.s2;
+        }
+    }
 }
 #endif
 template <class V>
