@@ -101,6 +101,7 @@ struct lg_ctx {
     CUfunction f_setp = nullptr, f_rraw = nullptr, f_rchi2 = nullptr, f_rdump = nullptr;
     CUfunction f_setp_split = nullptr;  // small batches: one warp per object
     int nobj = 0;
+    int sms = 148;
     CUfunction f_cchi2 = nullptr, f_cdump = nullptr;
     size_t model_bytes = 0;
     int rtiles = 0, ctiles = 0, ctiles_x = 0, ctiles_y = 0, cthreads = 0, csmem = 0;
@@ -185,6 +186,17 @@ struct lg_ctx {
                      : launch(f_setp, dim3((B + 127) / 128), dim3(128), 0, s, a_setp, "set_params");
     }
 
+    // Candidates one render block takes in turn: 1 where the program keeps
+    // no tables in shared memory; else up to 8 (its copy of the function
+    // tables is then below a percent of its work even for 9-point rules),
+    // fewer when that would leave less than 16 waves of 1024 threads per SM.
+    int render_per(int B) const
+    {
+        if (!lg::crf_in_smem(shape, lg::fp_mode(flags))) return 1;
+        const long blocks = (long)rtiles * B, wave = (long)sms * (1024 / shape.rt ? 1024 / shape.rt : 1);
+        return (int)std::max(1L, std::min(8L, blocks / (16 * wave)));
+    }
+
     // set = false: the object data are already in d_models
     int enqueue(int B, const double* params, double* logL, cudaStream_t s, cudaEvent_t* ev = nullptr,
                 bool set = true)
@@ -192,10 +204,11 @@ struct lg_ctx {
         int rc;
         auto mark = [&](int i) { return ev ? cuda(cudaEventRecord(ev[i], s), "event") : LG_OK; };
         if ((rc = mark(0)) || (set && (rc = launch_set(B, params, s))) || (rc = mark(1))) return rc;
+        int per = render_per(B);
+        const dim3 rgrid(rtiles, (B + per - 1) / per);
         if (psf) {
-            void* a_r[] = {&d_models, &d_raw};
-            if ((rc = launch(f_rraw, dim3(rtiles, B), dim3(shape.rt), 0, s, a_r, "render")) || (rc = mark(2)))
-                return rc;
+            void* a_r[] = {&d_models, &d_raw, &B, &per};
+            if ((rc = launch(f_rraw, rgrid, dim3(shape.rt), 0, s, a_r, "render")) || (rc = mark(2))) return rc;
             void* a_c[] = {&d_raw, &d_image, &d_weight, &d_partials, &d_counters, &logL};
             if ((rc = launch(f_cchi2, dim3(ctiles_x, ctiles_y, B), dim3(shape.ctx / shape.cr, shape.conv_block_y()),
                              csmem, s, a_c, "convolve")) ||
@@ -203,9 +216,8 @@ struct lg_ctx {
                 return rc;
             return mark(4);
         }
-        void* a_r[] = {&d_models, &d_image, &d_weight, &d_partials, &d_counters, &logL};
-        if ((rc = launch(f_rchi2, dim3(rtiles, B), dim3(shape.rt), 0, s, a_r, "render")) || (rc = mark(2)) ||
-            (rc = mark(3)))
+        void* a_r[] = {&d_models, &d_image, &d_weight, &d_partials, &d_counters, &logL, &B, &per};
+        if ((rc = launch(f_rchi2, rgrid, dim3(shape.rt), 0, s, a_r, "render")) || (rc = mark(2)) || (rc = mark(3)))
             return rc;
         return mark(4);
     }
@@ -609,6 +621,7 @@ int create_impl(lg_ctx* c, const lg_image_desc* img, const lg_object_desc* objs,
 
     if ((rc = c->cuda(cudaSetDevice(c->device), "cudaSetDevice"))) return rc;
     if ((rc = c->cuda(cudaFree(nullptr), "CUDA context"))) return rc;
+    cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device);
     c->drv = driver();
     if (!c->drv) return c->fail(LG_ERR_CUDA, "CUDA driver entry points unavailable");
     if ((rc = c->drvcall(c->drv->moduleLoadData(&c->mod_set, cubin_set.data()), "cuModuleLoadData"))) return rc;

@@ -175,6 +175,10 @@ inline bool fp_fmad(Fp m) { return m == Fp::FAST; }
 // LG_FLAG_IEEE_DIV)
 bool fp_ieee(int flags);
 
+// the evaluation module keeps the tables of the correctly rounded functions
+// in shared memory
+bool crf_in_smem(const Shape& s, Fp mode);
+
 // Compose the NVRTC sources of a model and compile them to cubins for
 // sm_103a.  The set_params module always uses the double-evaluated
 // elementary functions and no FMA contraction; the evaluation module per

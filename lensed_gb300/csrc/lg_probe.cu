@@ -11,6 +11,7 @@
 
 #include "lg_internal.h"
 #include "../device/lg_prelude.cuh"
+#define LG_CRF_SMEM 1
 #include "../device/lg_crfloat.cuh"
 
 namespace {
@@ -70,6 +71,7 @@ __device__ float crf_two_double(int fn, float x, unsigned u)
 __global__ void lg_crf_sweep_kernel(int fn, unsigned long long lo, unsigned long long hi,
                                     unsigned long long* __restrict__ bad, unsigned* __restrict__ first, int nfirst)
 {
+    crf_load_tables<256>(threadIdx.x);
     const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
     unsigned long long nbad = 0;
     for (unsigned long long u = lo + blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; u < hi; u += stride) {
@@ -102,6 +104,7 @@ __global__ void lg_crf_sweep_kernel(int fn, unsigned long long lo, unsigned long
 
 __global__ void lg_pair_math_kernel(int fn, const float* __restrict__ x, int n, float* __restrict__ out)
 {
+    crf_load_tables<256>(threadIdx.x);
     const int i = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
     if (i >= n) return;
     const lg_pair a = lg_pair_of(x[i], i + 1 < n ? x[i + 1] : 1.0f);

@@ -201,15 +201,24 @@ const char* mode_name(Fp mode) { return mode == Fp::FAST ? "fast" : (mode == Fp:
 // module and the strict and exact evaluation modules map the plugins'
 // float functions to the double-evaluated ones; the exact modules add the
 // correctly rounded single-precision functions and their ray-pair overloads.
-void emit_prelude(std::ostringstream& o, Fp mode, bool set)
+void emit_prelude(std::ostringstream& o, Fp mode, bool set, const Shape& s)
 {
-    if (!set && mode == Fp::EXACT) o << "#define LG_EXACT 1\n";
+    if (!set && mode == Fp::EXACT) {
+        o << "#define LG_EXACT 1\n";
+        if (crf_in_smem(s, mode)) o << "#define LG_CRF_SMEM 1\n";
+    }
     o << "\n" << prelude_source() << "\n";
     if (set || mode != Fp::FAST) o << crmath_source() << "\n";
     if (!set && mode == Fp::EXACT) o << crf_source() << "\n" << exact_pair_source() << "\n";
 }
 
 }  // namespace
+
+// The exact modules keep the tables of the correctly rounded functions
+// (24.6 KB) in shared memory, unless the values a quadrature split gathers
+// there (one point of each thread at least) leave too little of the 48 KB a
+// block may declare.
+bool crf_in_smem(const Shape& s, Fp mode) { return mode == Fp::EXACT && (s.qs == 1 || 4 * s.rt * s.rppt <= 22 * 1024); }
 
 std::string compose_source(const Model& m, const Shape& s, Fp mode, Part part)
 {
@@ -224,7 +233,7 @@ std::string compose_source(const Model& m, const Shape& s, Fp mode, Part part)
     o << "#define LG_CTX " << s.ctx << "\n#define LG_CTY " << s.cty << "\n#define LG_CR " << s.cr << "\n";
     // the paired modes with a PSF up to 49 wide pair rows unless the shape says not
     if (!strict && !s.pair_rows && m.psfw <= 49) o << "#define LG_CONV_SINGLE 1\n";
-    emit_prelude(o, mode, set);
+    emit_prelude(o, mode, set, s);
     std::set<std::string> done;
     for (const auto& ob : m.objs) emit_plugin(o, ob.plugin, done);
 
@@ -289,7 +298,7 @@ std::string compose_multi_source(const Model& m, const std::vector<std::pair<int
     o << "\n// rule " << m.rule->name << " (" << m.rule->size << " points), " << mode_name(mode) << " FP\n\n";
     o << "#define LG_RT " << s.rt << "\n#define LG_RPPT " << s.rppt << "\n#define LG_QS " << s.qs << "\n";
     o << "#define LG_CTX " << s.ctx << "\n#define LG_CTY " << s.cty << "\n#define LG_CR " << s.cr << "\n";
-    emit_prelude(o, mode, false);
+    emit_prelude(o, mode, false, s);
     std::set<std::string> done;
     for (const auto& ob : m.objs) emit_plugin(o, ob.plugin, done);
     o << "// ---- model section\n#define LG_NPARS " << m.pars.size() << "\n";

@@ -39,6 +39,10 @@
 #define LG_RTILES ((LG_N + LG_RTILE - 1) / LG_RTILE)
 static_assert(LG_QS == 1 || LG_QS == 2 || LG_QS == 4 || LG_QS == 8, "quadrature split of 1, 2, 4 or 8 threads");
 static_assert(LG_RT % 32 == 0, "render block of whole warps");
+// values a thread gathers at a time for the ordered sum: at most 16 KB a block
+#define LG_FQK_FIT (16384 / (LG_RT * LG_RPPT * 4))
+#define LG_FQK_ALL ((LG_Q + LG_QS - 1) / LG_QS)
+#define LG_FQK (LG_FQK_FIT < 1 ? 1 : (LG_FQK_FIT < LG_FQK_ALL ? LG_FQK_FIT : LG_FQK_ALL))
 
 // ------------------------------------------------------------ reductions --
 LG_DEV double lg_warp_sum(double v)
@@ -99,8 +103,10 @@ LG_DEV void lg_tile_done(double s, double* __restrict__ partials, int ntiles, in
 }
 
 // ---------------------------------------------------------------- render --
-// kernel/lensed.cl:9-39.  Block (tile, candidate); each group of LG_QS
-// threads integrates LG_RPPT pixels over the quadrature rule: strided by the
+// kernel/lensed.cl:9-39.  Block (tile, candidate), or in the exact modules
+// (tile, `per` candidates one after the other: the tables of the correctly
+// rounded functions are copied to shared memory once for all of them); each
+// group of LG_QS threads integrates LG_RPPT pixels over the quadrature rule: strided by the
 // group count in the scalar kernel (so that loads and stores coalesce),
 // adjacent in the paired kernel (a thread's two rays are neighbours, so they
 // mostly take the same branches; stores are float2).  With LG_QS > 1 the
@@ -126,9 +132,8 @@ template <int MODE>
 LG_DEV void lg_render_tile(const lg_model* __restrict__ models, float* __restrict__ out, float* __restrict__ err,
                            const float* __restrict__ image, const float* __restrict__ weight,
                            double* __restrict__ partials, unsigned* __restrict__ counters,
-                           double* __restrict__ logL)
+                           double* __restrict__ logL, int b)
 {
-    const int b = blockIdx.y;
     const lg_model m = models[b];
     const int base = blockIdx.x * LG_RTILE;
     const int grp = threadIdx.x / LG_QS, sub = threadIdx.x % LG_QS;
@@ -155,26 +160,32 @@ LG_DEV void lg_render_tile(const lg_model* __restrict__ models, float* __restric
     }
 #if defined(LG_EXACT) && LG_QS > 1
     // exact mode with a quadrature split: the threads of a group evaluate
-    // every LG_QS-th point, the values meet in shared memory, and every
-    // lane of the group sums all of them in the rule's order -- the sum the
-    // unsplit kernel forms, bit for bit
-    __shared__ float2 lg_fq[LG_RT][(LG_Q + LG_QS - 1) / LG_QS][LG_RPPT / 2];
+    // every LG_QS-th point, the values meet in shared memory (LG_FQK points
+    // a thread at a time), and every lane of the group sums all of them in
+    // the rule's order -- the sum the unsplit kernel forms, bit for bit
+    __shared__ float2 lg_fq[LG_RT][LG_FQK][LG_RPPT / 2];
 #pragma unroll 1
-    for (int n = sub, kq = 0; n < LG_Q; n += LG_QS, ++kq) {
-        const float2 q = lg_qq[n];
-#pragma unroll
-        for (int j = 0; j < LG_RPPT / 2; ++j) lg_fq[threadIdx.x][kq][j] = lg_compute2(m, lg_pair2{px[j] + q.x, py[j] + q.y}).v;
-    }
-    __syncwarp();
+    for (int n0 = 0; n0 < LG_Q; n0 += LG_QS * LG_FQK) {
+        __syncwarp();  // the reads of the values before are done
 #pragma unroll 1
-    for (int n = 0; n < LG_Q; ++n) {
-        const float2 w = lg_ww[n];
-        const int src = grp * LG_QS + n % LG_QS;
+        for (int n = n0 + sub, kq = 0; kq < LG_FQK && n < LG_Q; n += LG_QS, ++kq) {
+            const float2 q = lg_qq[n];
 #pragma unroll
-        for (int j = 0; j < LG_RPPT / 2; ++j) {
-            const lg_pair f = {lg_fq[src][n / LG_QS][j]};
-            pv[j] += w.x * f;
-            if (MODE == 2) pe[j] += w.y * f;
+            for (int j = 0; j < LG_RPPT / 2; ++j)
+                lg_fq[threadIdx.x][kq][j] = lg_compute2(m, lg_pair2{px[j] + q.x, py[j] + q.y}).v;
+        }
+        __syncwarp();
+        const int n1 = n0 + LG_QS * LG_FQK < LG_Q ? n0 + LG_QS * LG_FQK : LG_Q;
+#pragma unroll 1
+        for (int n = n0; n < n1; ++n) {
+            const float2 w = lg_ww[n];
+            const int src = grp * LG_QS + (n - n0) % LG_QS;
+#pragma unroll
+            for (int j = 0; j < LG_RPPT / 2; ++j) {
+                const lg_pair f = {lg_fq[src][(n - n0) / LG_QS][j]};
+                pv[j] += w.x * f;
+                if (MODE == 2) pe[j] += w.y * f;
+            }
         }
     }
 #else
@@ -257,6 +268,27 @@ LG_DEV void lg_render_tile(const lg_model* __restrict__ models, float* __restric
     }
 }
 
+// the block's candidates: blockIdx.y, or with the tables in shared memory
+// blockIdx.y per .. + per - 1 below B
+template <int MODE>
+LG_DEV void lg_render_block(const lg_model* __restrict__ models, float* __restrict__ out, float* __restrict__ err,
+                            const float* __restrict__ image, const float* __restrict__ weight,
+                            double* __restrict__ partials, unsigned* __restrict__ counters,
+                            double* __restrict__ logL, int B, int per)
+{
+#ifdef LG_CRF_SMEM
+    crf_load_tables<LG_RT>(threadIdx.x);
+    const int b0 = (int)blockIdx.y * per, b1 = b0 + per < B ? b0 + per : B;
+#pragma unroll 1
+    for (int b = b0; b < b1; ++b)
+        lg_render_tile<MODE>(models, out, err, image, weight, partials, counters, logL, b);
+#else
+    (void)B;
+    (void)per;
+    lg_render_tile<MODE>(models, out, err, image, weight, partials, counters, logL, blockIdx.y);
+#endif
+}
+
 // exact modules: 1024 resident threads per SM (64 registers a thread) --
 // the correctly rounded functions are issue-bound, and the extra warps hide
 // their latencies better than the 80 registers the compiler would use
@@ -266,23 +298,24 @@ LG_DEV void lg_render_tile(const lg_model* __restrict__ models, float* __restric
 #define LG_RENDER_MINB 1
 #endif
 extern "C" __global__ void __launch_bounds__(LG_RT, LG_RENDER_MINB) lg_render_raw(const lg_model* __restrict__ models,
-                                                                                  float* __restrict__ raw)
+                                                                                  float* __restrict__ raw, int B,
+                                                                                  int per)
 {
-    lg_render_tile<0>(models, raw, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
+    lg_render_block<0>(models, raw, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, B, per);
 }
 
 extern "C" __global__ void __launch_bounds__(LG_RT, LG_RENDER_MINB)
     lg_render_chi2(const lg_model* __restrict__ models, const float* __restrict__ image,
                    const float* __restrict__ weight, double* __restrict__ partials, unsigned* __restrict__ counters,
-                   double* __restrict__ logL)
+                   double* __restrict__ logL, int B, int per)
 {
-    lg_render_tile<1>(models, nullptr, nullptr, image, weight, partials, counters, logL);
+    lg_render_block<1>(models, nullptr, nullptr, image, weight, partials, counters, logL, B, per);
 }
 
 extern "C" __global__ void __launch_bounds__(LG_RT)
     lg_render_dump(const lg_model* __restrict__ models, float* __restrict__ value, float* __restrict__ error)
 {
-    lg_render_tile<2>(models, value, error, nullptr, nullptr, nullptr, nullptr, nullptr);
+    lg_render_block<2>(models, value, error, nullptr, nullptr, nullptr, nullptr, nullptr, 1, 1);
 }
 
 // -------------------------------------------------------------- convolve --

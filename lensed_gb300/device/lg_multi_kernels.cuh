@@ -25,6 +25,10 @@
 #define LG_RTILE (LG_RG * LG_RPPT)
 static_assert(LG_QS == 1 || LG_QS == 2 || LG_QS == 4 || LG_QS == 8, "quadrature split of 1, 2, 4 or 8 threads");
 static_assert(LG_RT % 32 == 0, "render block of whole warps");
+// values a thread gathers at a time for the ordered sum: at most 16 KB a block
+#define LG_FQK_FIT (16384 / (LG_RT * LG_RPPT * 4))
+#define LG_FQK_ALL ((LG_Q + LG_QS - 1) / LG_QS)
+#define LG_FQK (LG_FQK_FIT < 1 ? 1 : (LG_FQK_FIT < LG_FQK_ALL ? LG_FQK_FIT : LG_FQK_ALL))
 #ifndef LG_CTX
 #define LG_CTX 32
 #endif
@@ -111,6 +115,9 @@ LG_DEV void lg_multi_render_body(const lg_model* __restrict__ models, const lg_s
     __shared__ double red[LG_RT / 32];
     const long long U = hdr[0];
     const int nsys = (int)hdr[3];
+#ifdef LG_CRF_SMEM
+    crf_load_tables<LG_RT>(threadIdx.x);
+#endif
     const int grp = threadIdx.x / LG_QS, sub = threadIdx.x % LG_QS;
     for (long long u = blockIdx.x; u < U; u += gridDim.x) {
         const int s = lg_find_system(plan, nsys, u, false);
@@ -141,22 +148,26 @@ LG_DEV void lg_multi_render_body(const lg_model* __restrict__ models, const lg_s
 #if defined(LG_EXACT) && LG_QS > 1
         // exact mode with a quadrature split: values gathered in shared
         // memory and summed in the rule's order (as the single-system kernel)
-        __shared__ float2 lg_fq[LG_RT][(LG_Q + LG_QS - 1) / LG_QS][LG_RPPT / 2];
-        __syncwarp();  // the previous unit's reads of lg_fq are done
+        __shared__ float2 lg_fq[LG_RT][LG_FQK][LG_RPPT / 2];
 #pragma unroll 1
-        for (int n = sub, kq = 0; n < LG_Q; n += LG_QS, ++kq) {
-            const float2 q = lg_qq[n];
-#pragma unroll
-            for (int j = 0; j < LG_RPPT / 2; ++j)
-                lg_fq[threadIdx.x][kq][j] = lg_compute2(m, lg_pair2{px[j] + q.x, py[j] + q.y}).v;
-        }
-        __syncwarp();
+        for (int n0 = 0; n0 < LG_Q; n0 += LG_QS * LG_FQK) {
+            __syncwarp();  // the reads of the values before are done
 #pragma unroll 1
-        for (int n = 0; n < LG_Q; ++n) {
-            const float2 w = lg_ww[n];
-            const int src = grp * LG_QS + n % LG_QS;
+            for (int n = n0 + sub, kq = 0; kq < LG_FQK && n < LG_Q; n += LG_QS, ++kq) {
+                const float2 q = lg_qq[n];
 #pragma unroll
-            for (int j = 0; j < LG_RPPT / 2; ++j) pv[j] += w.x * lg_pair{lg_fq[src][n / LG_QS][j]};
+                for (int j = 0; j < LG_RPPT / 2; ++j)
+                    lg_fq[threadIdx.x][kq][j] = lg_compute2(m, lg_pair2{px[j] + q.x, py[j] + q.y}).v;
+            }
+            __syncwarp();
+            const int n1 = n0 + LG_QS * LG_FQK < LG_Q ? n0 + LG_QS * LG_FQK : LG_Q;
+#pragma unroll 1
+            for (int n = n0; n < n1; ++n) {
+                const float2 w = lg_ww[n];
+                const int src = grp * LG_QS + (n - n0) % LG_QS;
+#pragma unroll
+                for (int j = 0; j < LG_RPPT / 2; ++j) pv[j] += w.x * lg_pair{lg_fq[src][(n - n0) / LG_QS][j]};
+            }
         }
 #else
 #pragma unroll 1
