@@ -186,6 +186,14 @@ struct lg_ctx {
                      : launch(f_setp, dim3((B + 127) / 128), dim3(128), 0, s, a_setp, "set_params");
     }
 
+    // grid and block of the convolution: one block a tile, or 8 blocks of 128
+    // threads (32 x 8 outputs) a split tile
+    dim3 conv_grid(int B) const { return dim3(ctiles_x, ctiles_y * (shape.split_tiles ? 8 : 1), B); }
+    dim3 conv_block() const
+    {
+        return shape.split_tiles ? dim3(16, 8) : dim3(shape.ctx / shape.cr, shape.conv_block_y());
+    }
+
     // Candidates one render block takes in turn: 1 where the program keeps
     // no tables in shared memory; else up to 8 (its copy of the function
     // tables is then below a percent of its work even for 9-point rules),
@@ -210,8 +218,7 @@ struct lg_ctx {
             void* a_r[] = {&d_models, &d_raw, &B, &per};
             if ((rc = launch(f_rraw, rgrid, dim3(shape.rt), 0, s, a_r, "render")) || (rc = mark(2))) return rc;
             void* a_c[] = {&d_raw, &d_image, &d_weight, &d_partials, &d_counters, &logL};
-            if ((rc = launch(f_cchi2, dim3(ctiles_x, ctiles_y, B), dim3(shape.ctx / shape.cr, shape.conv_block_y()),
-                             csmem, s, a_c, "convolve")) ||
+            if ((rc = launch(f_cchi2, conv_grid(B), conv_block(), csmem, s, a_c, "convolve")) ||
                 (rc = mark(3)))
                 return rc;
             return mark(4);
@@ -277,7 +284,8 @@ namespace {
 
 // Launch shape for a model (tile sizes chosen for GB300; see the design
 // notes for the measurements behind them).
-lg::Shape choose_shape(const lg::Model& m, lg::Fp mode)
+// max_batch: the context's largest batch (0: many).
+lg::Shape choose_shape(const lg::Model& m, lg::Fp mode, int max_batch = 0)
 {
     lg::Shape s;
     // fast and exact modes: 32 x 64 convolution tiles, each thread two rows
@@ -286,6 +294,15 @@ lg::Shape choose_shape(const lg::Model& m, lg::Fp mode)
     if (!m.psf.empty() && mode != lg::Fp::STRICT && m.psfw <= 49) {
         s.cty = 64;
         s.pair_rows = true;
+    }
+    // a context for few candidates: its convolution tiles split over clusters
+    // and (exact mode, whose split sums in order) its quadrature over 2 or 4
+    // threads while that fills the GPU (lg::kSplitTiles, kSplitRays)
+    if (max_batch > 0 && s.pair_rows) {
+        const long tiles = (long)((m.width + 31) / 32) * ((m.height + 63) / 64) * max_batch;
+        if (tiles <= lg::kSplitTiles) s.split_tiles = true;
+        const long pairs = (long)m.width * m.height / 2 * max_batch;
+        while (mode == lg::Fp::EXACT && s.qs < 4 && s.qs < m.rule->size && pairs * s.qs * 2 <= lg::kSplitRays) s.qs *= 2;
     }
     return s;
 }
@@ -297,7 +314,7 @@ void shape_sizes(const lg::Shape& s, const lg::Model& m, lg_ctx* c)
     c->rtiles = (int)((N + rtile - 1) / rtile);
     if (!m.psf.empty()) {
         // the shared-memory size is read back from the compiled module
-        c->cthreads = (s.ctx / s.cr) * s.conv_block_y();
+        c->cthreads = s.split_tiles ? 128 : (s.ctx / s.cr) * s.conv_block_y();
         c->ctiles_x = (m.width + s.ctx - 1) / s.ctx;
         c->ctiles_y = (m.height + s.cty - 1) / s.cty;
         c->ctiles = c->ctiles_x * c->ctiles_y;
@@ -613,7 +630,7 @@ int create_impl(lg_ctx* c, const lg_image_desc* img, const lg_object_desc* objs,
     // src/lensed.c:706-776): the set_params module here, the evaluation
     // module (whose launch shape may be tuned) once the buffers exist
     const lg::Fp mode = lg::fp_mode(c->flags);
-    c->shape = choose_shape(m, mode);
+    c->shape = choose_shape(m, mode, c->max_batch);
     std::string log;
     std::vector<char> cubin_set;
     rc = lg::compile_program(lg::compose_source(m, c->shape, mode, lg::Part::SET), false, cubin_set, log);
@@ -1322,9 +1339,7 @@ int render_device(lg_ctx* c, const double* params, const float** d_model)
     if ((rc = c->launch(c->f_rdump, dim3(c->rtiles, 1), dim3(c->shape.rt), 0, c->stream, a_r, "render"))) return rc;
     if (c->psf) {
         void* a_c[] = {&d_val, &c->d_raw};
-        if ((rc = c->launch(c->f_cdump, dim3(c->ctiles_x, c->ctiles_y, 1),
-                            dim3(c->shape.ctx / c->shape.cr, c->shape.conv_block_y()),
-                            c->csmem, c->stream, a_c, "convolve")))
+        if ((rc = c->launch(c->f_cdump, c->conv_grid(1), c->conv_block(), c->csmem, c->stream, a_c, "convolve")))
             return rc;
     }
     *d_model = c->psf ? c->d_raw : d_val;

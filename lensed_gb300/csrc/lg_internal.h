@@ -148,12 +148,13 @@ struct Shape {
     int qs = 1;                    // threads per group splitting the quadrature points
     int ctx = 32, cty = 32, cr = 8; // convolution tile and outputs per thread
     bool pair_rows = false;        // convolution threads own two rows (f32x2)
+    bool split_tiles = false;      // each paired tile over a cluster of blocks (same result, few tiles)
     int conv_block_y() const { return pair_rows ? cty / 2 : cty; }
     int rtile() const { return rt / qs * rppt; }  // pixels per render block
     bool operator==(const Shape& o) const
     {
         return rt == o.rt && rppt == o.rppt && qs == o.qs && ctx == o.ctx && cty == o.cty && cr == o.cr &&
-               pair_rows == o.pair_rows;
+               pair_rows == o.pair_rows && split_tiles == o.split_tiles;
     }
     std::string str() const;
 };
@@ -178,6 +179,18 @@ bool fp_ieee(int flags);
 // the evaluation module keeps the tables of the correctly rounded functions
 // in shared memory
 bool crf_in_smem(const Shape& s, Fp mode);
+
+// A context whose largest batch has at most kSplitTiles convolution tiles
+// splits each over a cluster of 8 blocks: 608 blocks then fill 152 SMs.
+// Convolution stage, whole against split tiles (us): 256^2, 25^2 PSF, 32 tiles
+// 22.5 / 16.3, 64 tiles 24.5 / 20.5, 128 tiles 22.5 / 28.7; 64^2, 17^2 PSF, 32
+// tiles 20.4 / 12.2, 64 tiles 20.5 / 16.4, 128 tiles 20.4 / 20.4.
+// With a split quadrature while the threads stay below kSplitRays (1024 an
+// SM), render stage, unsplit / 2 / 4 threads (us): 256^2, 25 points, 1
+// candidate 40.4 / 30.2 / 28.1, 2 candidates 48.7 / 46.6 / 46.6, 4 candidates
+// 81.4 / 81.4 / 82.5; 101 x 77, 25 points, 7 candidates 19.1 / 15.9 / 15.8, 16
+// candidates 23.2 / 24.0 / 24.2.
+constexpr long kSplitTiles = 76, kSplitRays = 152 * 1024;
 
 // Compose the NVRTC sources of a model and compile them to cubins for
 // sm_103a.  The set_params module always uses the double-evaluated

@@ -233,6 +233,7 @@ std::string compose_source(const Model& m, const Shape& s, Fp mode, Part part)
     o << "#define LG_CTX " << s.ctx << "\n#define LG_CTY " << s.cty << "\n#define LG_CR " << s.cr << "\n";
     // the paired modes with a PSF up to 49 wide pair rows unless the shape says not
     if (!strict && !s.pair_rows && m.psfw <= 49) o << "#define LG_CONV_SINGLE 1\n";
+    if (s.split_tiles) o << "#define LG_CONV_SPLIT 1\n";
     emit_prelude(o, mode, set, s);
     std::set<std::string> done;
     for (const auto& ob : m.objs) emit_plugin(o, ob.plugin, done);
@@ -276,7 +277,8 @@ std::string compose_source(const Model& m, const Shape& s, Fp mode, Part part)
     o << "};\n";
     if (!m.psf.empty()) {
         o << "#define LG_HAS_PSF 1\n#define LG_PSF_W " << m.psfw << "\n#define LG_PSF_H " << m.psfh << "\n";
-        o << "__constant__ float lg_psf[LG_PSF_W * LG_PSF_H] = {";
+        // (the split tiles stage the PSF in shared memory)
+        o << (s.split_tiles ? "__device__ const" : "__constant__") << " float lg_psf[LG_PSF_W * LG_PSF_H] = {";
         for (size_t i = 0; i < m.psf.size(); ++i) o << (i ? (i % 8 ? ", " : ",\n    ") : "") << hexf(m.psf[i]);
         o << "};\n";
     } else {

@@ -365,7 +365,149 @@ LG_DEV double lg_conv_out(int b, int gy, int gx0, const float* acc, float* __res
     return s;
 }
 
-#if defined(LG_PAIRED) && LG_PSF_W <= 49 && !defined(LG_CONV_SINGLE)
+#if defined(LG_CONV_SPLIT)
+// Few tiles (contexts of one or a few candidates): the 32 x 64 tile of the
+// paired kernel below, split over a cluster of 8 blocks of 32 x 8 outputs, 128
+// threads of 2 outputs each -- one image of 256^2 then fills 256 blocks
+// instead of 32.  What bounds it is latency: the halo and PSF loads (the PSF
+// through shared memory: a cold constant cache costs a miss per 64 bytes), PW
+// x PH dependent adds, and the FP64 sums.  Each block sums its rows' chi^2
+// terms as the paired kernel's threads do (8 columns of a row in order); the
+// row sums of all 8 meet in the first block's shared memory, which adds them
+// up in that kernel's grouping, so logL is the same bit for bit whatever the
+// batch size the context was made for.
+#define LG_CSPLIT 8
+#define LG_CTHREADS 128
+#define LG_SROWS (LG_CTY / LG_CSPLIT)
+#define LG_SWIN ((2 + LG_PSF_W - 1 + 1) / 2 * 2)
+#define LG_SPITCH (LG_CTX - 2 + LG_SWIN)
+#define LG_SHALO (LG_SROWS + LG_PSF_H - 1)
+#define LG_SPSFW ((LG_PSF_W + 3) / 4 * 4)
+#define LG_CSMEM ((LG_PSF_H * LG_SPSFW + LG_SHALO * LG_SPITCH) * 4)
+static_assert(LG_CTX == 32 && LG_CTY == 64 && LG_CR == 8, "the split tile is the default paired one");
+
+// address of `p` in the shared memory of the cluster's first block
+LG_DEV unsigned lg_first_block(const void* p)
+{
+    unsigned a;
+    asm("{\n.reg .u64 t;\n.reg .u32 s;\ncvta.to.shared.u64 t, %1;\ncvt.u32.u64 s, t;\n"
+        "mapa.shared::cluster.u32 %0, s, 0;\n}"
+        : "=r"(a)
+        : "l"(p));
+    return a;
+}
+LG_DEV void lg_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+LG_DEV void lg_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+template <int MODE>
+LG_DEV void lg_conv_tile(const float* __restrict__ raw, float* __restrict__ out, const float* __restrict__ image,
+                         const float* __restrict__ weight, double* __restrict__ partials,
+                         unsigned* __restrict__ counters, double* __restrict__ logL)
+{
+    extern __shared__ float4 lg_smem4[];
+    float* psf = reinterpret_cast<float*>(lg_smem4);
+    float* tile = psf + LG_PSF_H * LG_SPSFW;
+    if (MODE == 1) lg_cluster_arrive();  // every block of the cluster has started
+    const int b = blockIdx.z;
+    const float* src = raw + (size_t)b * LG_N;
+    const int X0 = blockIdx.x * LG_CTX, Y0 = blockIdx.y * LG_SROWS;
+    const int tid = threadIdx.y * 16 + threadIdx.x;
+    const int lx0 = threadIdx.x * 2, ly = threadIdx.y;
+    const int gy = Y0 + ly, gx0 = X0 + lx0;
+    float d[2] = {0.0f, 0.0f}, w[2] = {0.0f, 0.0f};
+    bool in[2];
+#pragma unroll
+    for (int o = 0; o < 2; ++o) {
+        in[o] = gy < LG_H && gx0 + o < LG_W;
+        if (MODE == 1 && in[o]) {
+            d[o] = image[gy * LG_W + gx0 + o];
+            w[o] = weight[gy * LG_W + gx0 + o];
+        }
+    }
+#pragma unroll 8
+    for (int i = tid; i < LG_PSF_H * LG_SPSFW; i += LG_CTHREADS) {
+        const int r = i / LG_SPSFW, c = i - r * LG_SPSFW;
+        psf[i] = c < LG_PSF_W ? lg_psf[r * LG_PSF_W + c] : 0.0f;
+    }
+    const int br = Y0 + LG_OY - (LG_PSF_H - 1), bc = X0 + LG_OX - (LG_PSF_W - 1);
+#pragma unroll 16
+    for (int i = tid; i < LG_SHALO * LG_SPITCH; i += LG_CTHREADS) {
+        const int r = i / LG_SPITCH, c = i - r * LG_SPITCH;
+        int sy = br + r, sx = bc + c;
+        sy = sy < 0 ? 0 : (sy > LG_H - 1 ? LG_H - 1 : sy);
+        sx = sx < 0 ? 0 : (sx > LG_W - 1 ? LG_W - 1 : sx);
+        tile[i] = src[sy * LG_W + sx];
+    }
+    __syncthreads();
+    float acc[2] = {0.0f, 0.0f};
+#pragma unroll 1
+    for (int j = 0; j < LG_PSF_H; ++j) {
+        float win[LG_SWIN], p[LG_SPSFW];
+        const float2* row = reinterpret_cast<const float2*>(tile + (ly + LG_PSF_H - 1 - j) * LG_SPITCH + lx0);
+        const float4* prow = reinterpret_cast<const float4*>(psf + j * LG_SPSFW);
+#pragma unroll
+        for (int t = 0; t < LG_SWIN / 2; ++t) {
+            const float2 q = row[t];
+            win[2 * t + 0] = q.x;
+            win[2 * t + 1] = q.y;
+        }
+#pragma unroll
+        for (int t = 0; t < LG_SPSFW / 4; ++t) {
+            const float4 q = prow[t];
+            p[4 * t + 0] = q.x;
+            p[4 * t + 1] = q.y;
+            p[4 * t + 2] = q.z;
+            p[4 * t + 3] = q.w;
+        }
+#pragma unroll
+        for (int i = 0; i < LG_PSF_W; ++i)
+#pragma unroll
+            for (int o = 0; o < 2; ++o) acc[o] += p[i] * win[o + LG_PSF_W - 1 - i];
+    }
+    if (MODE == 0) {
+#pragma unroll
+        for (int o = 0; o < 2; ++o)
+            if (in[o]) out[(size_t)b * LG_N + gy * LG_W + gx0 + o] = acc[o];
+        return;
+    }
+    // chi^2 terms (0 outside the image: the sum of the rest is unchanged), the
+    // sums of 8 columns of each of the block's rows, and those of the whole
+    // tile in the first block
+    __shared__ float2 terms[LG_SROWS * LG_CTX / 2];
+    __shared__ double rows[LG_CTY * LG_CTX / 8];
+    __shared__ double red[4];
+    float t[2];
+#pragma unroll
+    for (int o = 0; o < 2; ++o) {
+        const float e = acc[o] - d[o];
+        t[o] = in[o] ? w[o] * e * e : 0.0f;
+    }
+    terms[tid] = make_float2(t[0], t[1]);
+    __syncthreads();
+    lg_cluster_wait();
+    if (tid < 32) {
+        double s = 0.0;
+#pragma unroll
+        for (int o = 0; o < 4; ++o) {
+            const float2 q = terms[tid * 4 + o];
+            s += (double)q.x;
+            s += (double)q.y;
+        }
+        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(
+                         lg_first_block(rows + (blockIdx.y % LG_CSPLIT) * LG_SROWS * 4 + tid)),
+                     "d"(s)
+                     : "memory");
+    }
+    lg_cluster_arrive();
+    lg_cluster_wait();
+    if (blockIdx.y % LG_CSPLIT != 0) return;
+    // the paired kernel's thread (x, y): rows y and y + 32 of 8 columns
+    const double s = lg_block_sum<LG_CTHREADS>(rows[tid] + rows[tid + 128], red);
+    lg_tile_done<LG_CTHREADS>(s, partials, LG_CTILES, (blockIdx.y / LG_CSPLIT) * LG_CTILES_X + blockIdx.x, b, counters,
+                              logL, red);
+}
+#define LG_CONV_CLUSTER __cluster_dims__(1, LG_CSPLIT, 1)
+#elif defined(LG_PAIRED) && LG_PSF_W <= 49 && !defined(LG_CONV_SINGLE)
 // Paired rows (fast and exact modes, PSFs up to 49 pixels wide, unless the
 // launch shape asks for single rows -- small tiles for small batches): a
 // thread computes LG_CR columns of two output rows, y and y + LG_CTY/2, with
@@ -526,7 +668,10 @@ LG_DEV void lg_conv_tile(const float* __restrict__ raw, float* __restrict__ out,
 }
 #endif
 
-extern "C" __global__ void __launch_bounds__(LG_CTHREADS)
+#ifndef LG_CONV_CLUSTER
+#define LG_CONV_CLUSTER
+#endif
+extern "C" __global__ void LG_CONV_CLUSTER __launch_bounds__(LG_CTHREADS)
     lg_conv_chi2(const float* __restrict__ raw, const float* __restrict__ image, const float* __restrict__ weight,
                  double* __restrict__ partials, unsigned* __restrict__ counters, double* __restrict__ logL)
 {
