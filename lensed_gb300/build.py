@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import glob
 import os
+import re
 import subprocess
 import sys
 from concurrent.futures import ThreadPoolExecutor
@@ -33,6 +34,10 @@ def cuda_home() -> str:
 
 
 def _raw(text: str) -> str:
+    """A C++ raw string of device code without its comments (NVRTC reads the
+    text with every model it compiles)."""
+    text = re.sub(r"[ \t]*//[^\n]*", "", text)
+    text = re.sub(r"\n{2,}", "\n", text)
     assert ")LGRAW\"" not in text
     return 'R"LGRAW(' + text + ')LGRAW"'
 
@@ -44,12 +49,15 @@ def write_embed() -> str:
     setk = open(os.path.join(PKG, "device", "lg_set_kernel.cuh")).read()
     crmath = open(os.path.join(PKG, "device", "lg_crmath_on.cuh")).read()
     multi = open(os.path.join(PKG, "device", "lg_multi_kernels.cuh")).read()
-    # the correctly rounded functions with their tables inlined (NVRTC has no
-    # include path to this tree)
-    inc = '#ifndef LG_CRF_TABLES_INLINE\n#include "lg_crf_tables.cuh"\n#endif\n'
+    # the correctly rounded functions with their constants inlined (NVRTC has no
+    # include path to this tree; the tables stay in the library)
+    inc = '#ifndef LG_CRF_CONSTS_INLINE\n#include "lg_crf_consts.cuh"\n#endif\n'
     crf = open(os.path.join(PKG, "device", "lg_crfloat.cuh")).read()
     assert inc in crf
-    crf = crf.replace(inc, open(os.path.join(PKG, "device", "lg_crf_tables.cuh")).read())
+    crf = crf.replace(inc, open(os.path.join(PKG, "device", "lg_crf_consts.cuh")).read())
+    # without the quick phases for the set_params modules
+    crf_full = re.sub(r"#ifndef LG_CRF_NO_QUICK\n.*?#endif  // LG_CRF_NO_QUICK\n", "", crf, flags=re.S)
+    assert len(crf_full) < len(crf)
     exact = open(os.path.join(PKG, "device", "lg_exact_pair.cuh")).read()
     objs = sorted(glob.glob(os.path.join(PKG, "objects", "*.cuh")))
     lines = ["// generated by lensed_gb300/build.py: device sources for NVRTC", ""]
@@ -59,6 +67,7 @@ def write_embed() -> str:
     lines.append(f"static const char LG_EMBED_CRMATH[] = {_raw(crmath)};")
     lines.append(f"static const char LG_EMBED_MULTI[] = {_raw(multi)};")
     lines.append(f"static const char LG_EMBED_CRF[] = {_raw(crf)};")
+    lines.append(f"static const char LG_EMBED_CRF_FULL[] = {_raw(crf_full)};")
     lines.append(f"static const char LG_EMBED_EXACT_PAIR[] = {_raw(exact)};")
     lines.append("struct lg_embedded_object { const char* name; const char* text; };")
     lines.append("static const lg_embedded_object LG_EMBED_OBJECTS[] = {")

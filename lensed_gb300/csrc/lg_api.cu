@@ -99,8 +99,7 @@ struct lg_ctx {
     CUmodule mod = nullptr;      // evaluation module
     CUmodule mod_set = nullptr;  // set_params module
     CUfunction f_setp = nullptr, f_rraw = nullptr, f_rchi2 = nullptr, f_rdump = nullptr;
-    CUfunction f_setp_split = nullptr;  // small batches: one warp per object
-    int nobj = 0;
+    int set_shape[2] = {0, 0};  // candidates and threads of a set_params block
     int sms = 148;
     CUfunction f_cchi2 = nullptr, f_cdump = nullptr;
     size_t model_bytes = 0;
@@ -170,20 +169,11 @@ struct lg_ctx {
         return drvcall(drv->launchKernel(f, g.x, g.y, g.z, b.x, b.y, b.z, smem, (CUstream)s, args, nullptr), what);
     }
 
-    // Enqueue set_params, render and (with a PSF) convolve for B
-    // candidates; params and logL are device pointers (the last stage ends
-    // with logL, the block finishing a candidate's last tile summing its
-    // partials).  With ev != NULL, ev[0..4] are recorded before set_params,
-    // render, convolve and after the last stage (twice: no separate finish).
-    // set_params for B candidates into d_models: a handful of candidates
-    // get the objects of a candidate side by side (one warp each); else one
-    // thread per candidate
+    // set_params for B candidates into d_models
     int launch_set(int B, const double* params, cudaStream_t s)
     {
         void* a_setp[] = {&params, &B, &d_models};
-        const bool split = B <= 32 && nobj > 1 && nobj <= 32;
-        return split ? launch(f_setp_split, dim3(B), dim3(32 * nobj), 0, s, a_setp, "set_params")
-                     : launch(f_setp, dim3((B + 127) / 128), dim3(128), 0, s, a_setp, "set_params");
+        return launch(f_setp, dim3((B + set_shape[0] - 1) / set_shape[0]), dim3(set_shape[1]), 0, s, a_setp, "set_params");
     }
 
     // grid and block of the convolution: one block a tile, or 8 blocks of 128
@@ -205,6 +195,11 @@ struct lg_ctx {
         return (int)std::max(1L, std::min(8L, blocks / (16 * wave)));
     }
 
+    // Enqueue set_params, render and (with a PSF) convolve for B
+    // candidates; params and logL are device pointers (the last stage ends
+    // with logL, the block finishing a candidate's last tile summing its
+    // partials).  With ev != NULL, ev[0..4] are recorded before set_params,
+    // render, convolve and after the last stage (twice: no separate finish).
     // set = false: the object data are already in d_models
     int enqueue(int B, const double* params, double* logL, cudaStream_t s, cudaEvent_t* ev = nullptr,
                 bool set = true)
@@ -419,6 +414,7 @@ int load_eval(lg_ctx* c, const lg::Shape& s, const std::vector<char>& cubin)
     c->shape = s;
     shape_sizes(s, c->model, c);
     if ((rc = c->drvcall(c->drv->moduleLoadData(&c->mod, cubin.data()), "cuModuleLoadData"))) return rc;
+    if (ctx_mode(c) == lg::Fp::EXACT && (rc = lg::bind_crf_tables(c->mod, c->err))) return rc;
     struct {
         CUfunction* f;
         const char* n;
@@ -641,11 +637,11 @@ int create_impl(lg_ctx* c, const lg_image_desc* img, const lg_object_desc* objs,
     cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device);
     c->drv = driver();
     if (!c->drv) return c->fail(LG_ERR_CUDA, "CUDA driver entry points unavailable");
-    if ((rc = c->drvcall(c->drv->moduleLoadData(&c->mod_set, cubin_set.data()), "cuModuleLoadData"))) return rc;
+    if ((rc = c->drvcall(c->drv->moduleLoadData(&c->mod_set, cubin_set.data()), "cuModuleLoadData")) ||
+        (mode == lg::Fp::EXACT && (rc = lg::bind_crf_tables(c->mod_set, c->err))))
+        return rc;
     if ((rc = c->drvcall(c->drv->moduleGetFunction(&c->f_setp, c->mod_set, "lg_set_params_kernel"),
-                         "lg_set_params_kernel")) ||
-        (rc = c->drvcall(c->drv->moduleGetFunction(&c->f_setp_split, c->mod_set, "lg_set_params_split"),
-                         "lg_set_params_split")))
+                         "lg_set_params_kernel")))
         return rc;
     CUdeviceptr gp;
     size_t gb;
@@ -654,8 +650,8 @@ int create_impl(lg_ctx* c, const lg_image_desc* img, const lg_object_desc* objs,
     unsigned mb = 0;
     if ((rc = c->cuda(cudaMemcpy(&mb, (void*)gp, sizeof mb, cudaMemcpyDeviceToHost), "model size"))) return rc;
     c->model_bytes = mb;
-    if ((rc = c->drvcall(c->drv->moduleGetGlobal(&gp, &gb, c->mod_set, "lg_model_objects"), "lg_model_objects")) ||
-        (rc = c->cuda(cudaMemcpy(&c->nobj, (void*)gp, sizeof c->nobj, cudaMemcpyDeviceToHost), "object count")))
+    if ((rc = c->drvcall(c->drv->moduleGetGlobal(&gp, &gb, c->mod_set, "lg_set_shape"), "lg_set_shape")) ||
+        (rc = c->cuda(cudaMemcpy(c->set_shape, (void*)gp, sizeof c->set_shape, cudaMemcpyDeviceToHost), "set shape")))
         return rc;
 
     if ((rc = c->cuda(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking), "stream")) ||
@@ -1329,12 +1325,7 @@ int render_device(lg_ctx* c, const double* params, const float** d_model)
     float* d_val = c->d_model_out;
     if ((rc = c->cuda(cudaMemcpyAsync(c->d_params, params, np * 8, cudaMemcpyHostToDevice, c->stream), "params")))
         return rc;
-    int one = 1;
-    void* a_setp[] = {&c->d_params, &one, &c->d_models};
-    if ((rc = c->nobj > 1 && c->nobj <= 32
-                  ? c->launch(c->f_setp_split, dim3(1), dim3(32 * c->nobj), 0, c->stream, a_setp, "set_params")
-                  : c->launch(c->f_setp, dim3(1), dim3(128), 0, c->stream, a_setp, "set_params")))
-        return rc;
+    if ((rc = c->launch_set(1, c->d_params, c->stream))) return rc;
     void* a_r[] = {&c->d_models, &d_val, &c->d_err_out};
     if ((rc = c->launch(c->f_rdump, dim3(c->rtiles, 1), dim3(c->shape.rt), 0, c->stream, a_r, "render"))) return rc;
     if (c->psf) {

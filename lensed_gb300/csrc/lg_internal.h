@@ -59,7 +59,8 @@ const char* kernels_source();
 const char* set_kernel_source();
 const char* crmath_source();
 const char* multi_kernels_source();
-const char* crf_source();         // correctly rounded exp/log/atan/atanh in FP32 arithmetic
+const char* crf_source();       // correctly rounded functions in FP32 arithmetic
+const char* crf_full_source();  // the same without the quick phases of ray pairs
 const char* exact_pair_source();  // their ray-pair overloads for the exact modules
 
 // ------------------------------------------------------------------- priors
@@ -176,6 +177,9 @@ inline bool fp_fmad(Fp m) { return m == Fp::FAST; }
 // LG_FLAG_IEEE_DIV)
 bool fp_ieee(int flags);
 
+// an exact context's modules use the correctly rounded functions and need
+// the tables' address after loading
+int bind_crf_tables(CUmodule mod, std::string& err);
 // the evaluation module keeps the tables of the correctly rounded functions
 // in shared memory
 bool crf_in_smem(const Shape& s, Fp mode);

@@ -105,58 +105,27 @@ void emit_compute2(std::ostringstream& o, const Model& m)
 // object's own plane.
 void emit_set_params(std::ostringstream& o, const Model& m)
 {
-    o << "LG_DEV void lg_set_params(lg_model& m, const float* p)\n{\n"
-      << "    float2 x = make_float2(0.0f, 0.0f);\n    float2 a = make_float2(0.0f, 0.0f);\n"
-      << "    (void)x;\n    (void)a;\n";
     int trigger = 0;
     size_t plane = 0;
-    for (size_t i = 0; i < m.objs.size(); ++i) {
-        const ObjectInfo& ob = m.objs[i];
-        const Plugin* pl = ob.plugin;
-        if (pl->kind != trigger && pl->kind != LG_FOREGROUND) {
-            if (trigger == LG_LENS && pl->kind == LG_SOURCE) plane = i;
-            trigger = pl->kind;
-        }
-        const int np = (int)pl->pars.size();
-        if (ob.ipp) {
-            int xp = -1;
-            for (int j = 0; j < np; ++j)
-                if (m.pars[ob.par0 + j].prior.ipp && pl->pars[j].type == LG_POSITION_X) xp = j;
-            o << "    x = make_float2(p[" << ob.par0 + xp << "], p[" << ob.par0 + xp + 1 << "]);\n";
-            int trigger2 = 0;
-            for (size_t k = 0; k < plane; ++k) {
-                const Plugin* q = m.objs[k].plugin;
-                if (q->kind != trigger2 && q->kind != LG_FOREGROUND) {
-                    if (trigger2 == LG_LENS) o << "    lg_deflect(x, a);\n    a = make_float2(0.0f, 0.0f);\n";
-                    trigger2 = q->kind;
-                }
-                if (q->kind == LG_LENS) o << "    a += lg_deflection_" << q->name << "(&m.o" << k << ", x);\n";
-            }
-            if (trigger2 == LG_LENS) o << "    lg_deflect(x, a);\n    a = make_float2(0.0f, 0.0f);\n";
-        }
-        o << "    lg_set_" << pl->name << "(&m.o" << i;
-        for (int j = 0; j < np; ++j) {
-            const ParamInfo& pi = m.pars[ob.par0 + j];
-            if (ob.ipp && pi.prior.ipp)
-                o << ", " << (pl->pars[j].type == LG_POSITION_X ? "x.x" : (pl->pars[j].type == LG_POSITION_Y ? "x.y" : "0"));
-            else
-                o << ", p[" << ob.par0 + j << "]";
-        }
-        o << ");\n";
-    }
-    o << "}\n\n";
-    // the same, one object at a time (for the kernel that gives every object
-    // its own warp): objects with image-plane priors read the lenses of
-    // earlier planes, so they run in a second phase
+    // one object at a time: objects with image-plane priors behind a lens read
+    // the lenses of earlier planes, so they run in a second phase
     o << "#define LG_NOBJ " << m.objs.size() << "\n";
     o << "__constant__ int lg_obj_phase[LG_NOBJ] = {";
-    for (size_t i = 0; i < m.objs.size(); ++i) o << (i ? ", " : "") << (m.objs[i].ipp ? 1 : 0);
+    for (size_t i = 0; i < m.objs.size(); ++i) {
+        const int kind = m.objs[i].plugin->kind;
+        if (kind != trigger && kind != LG_FOREGROUND) {
+            if (trigger == LG_LENS && kind == LG_SOURCE) plane = i;
+            trigger = kind;
+        }
+        // (a lens's own image-plane position is deflected by nothing)
+        o << (i ? ", " : "") << (m.objs[i].ipp && plane > 0 ? 1 : 0);
+    }
     o << "};\n";
-    o << "LG_DEV void lg_set_object(lg_model& m, const float* p, int which)\n{\n"
-      << "    float2 x = make_float2(0.0f, 0.0f);\n    float2 a = make_float2(0.0f, 0.0f);\n"
-      << "    (void)x;\n    (void)a;\n    switch (which) {\n";
     trigger = 0;
     plane = 0;
+    o << "static __device__ __noinline__ void lg_set_object(lg_model& m, const float* p, int which)\n{\n"
+      << "    float2 x = make_float2(0.0f, 0.0f);\n    float2 a = make_float2(0.0f, 0.0f);\n"
+      << "    (void)x;\n    (void)a;\n    switch (which) {\n";
     for (size_t i = 0; i < m.objs.size(); ++i) {
         const ObjectInfo& ob = m.objs[i];
         const Plugin* pl = ob.plugin;
@@ -208,6 +177,11 @@ void emit_prelude(std::ostringstream& o, Fp mode, bool set, const Shape& s)
         if (crf_in_smem(s, mode)) o << "#define LG_CRF_SMEM 1\n";
     }
     o << "\n" << prelude_source() << "\n";
+    if (mode == Fp::EXACT) o << "#define LG_CRF_MODULE 1\n";
+    // (an exact context's set_params takes the single-precision functions too:
+    // the same values, 8 us less for a few candidates; reading their source
+    // takes NVRTC 6 ms, which the other modes' contexts would pay for less)
+    if (set && mode == Fp::EXACT) o << "#define LG_CRF_NO_QUICK 1\n" << crf_full_source() << "\n";
     if (set || mode != Fp::FAST) o << crmath_source() << "\n";
     if (!set && mode == Fp::EXACT) o << crf_source() << "\n" << exact_pair_source() << "\n";
 }

@@ -25,6 +25,7 @@ const char* set_kernel_source() { return LG_EMBED_SET_KERNEL; }
 const char* crmath_source() { return LG_EMBED_CRMATH; }
 const char* multi_kernels_source() { return LG_EMBED_MULTI; }
 const char* crf_source() { return LG_EMBED_CRF; }
+const char* crf_full_source() { return LG_EMBED_CRF_FULL; }
 const char* exact_pair_source() { return LG_EMBED_EXACT_PAIR; }
 
 namespace {

@@ -56,6 +56,7 @@ struct lg_systems {
     CUmodule mod = nullptr, mod_set = nullptr;
     CUfunction f_setp = nullptr, f_render = nullptr, f_conv = nullptr, f_finish = nullptr;
     int grid_render = 0, grid_conv = 0, grid_finish = 0, csmem = 0;
+    int set_shape[2] = {0, 0};  // candidates and threads of a set_params block
 
     cudaStream_t stream = nullptr;
     float *d_images = nullptr, *d_weights = nullptr, *d_psfs = nullptr, *d_raw = nullptr;
@@ -202,6 +203,7 @@ int apply_shape(lg_systems* S, const lg::Shape& sh, const std::vector<char>& cub
         return S->fail(LG_ERR_UNSUPPORTED, "convolution tile needs " + std::to_string(csmem) +
                                                " bytes of shared memory, above the device's " + std::to_string(optin));
     if ((rc = S->drvcall(S->drv->moduleLoadData(&S->mod, cubin.data()), "cuModuleLoadData")) ||
+        (sys_mode(S) == lg::Fp::EXACT && (rc = lg::bind_crf_tables(S->mod, S->err))) ||
         (rc = S->drvcall(S->drv->moduleGetFunction(&S->f_render, S->mod,
                                                    S->psf ? "lg_multi_render_raw" : "lg_multi_render_chi2"),
                          "render")) ||
@@ -337,13 +339,16 @@ int create_systems(lg_systems* S, const lg_image_desc* images, int nsys, const l
     S->drv = lg::driver();
     if (!S->drv) return S->fail(LG_ERR_CUDA, "CUDA driver entry points unavailable");
     if ((rc = S->drvcall(S->drv->moduleLoadData(&S->mod_set, cubin_set.data()), "cuModuleLoadData")) ||
+        (mode == lg::Fp::EXACT && (rc = lg::bind_crf_tables(S->mod_set, S->err))) ||
         (rc = S->drvcall(S->drv->moduleGetFunction(&S->f_setp, S->mod_set, "lg_set_params_kernel"), "set_params")))
         return rc;
     CUdeviceptr gp;
     size_t gb;
     unsigned mb = 0;
     if ((rc = S->drvcall(S->drv->moduleGetGlobal(&gp, &gb, S->mod_set, "lg_model_bytes"), "model size")) ||
-        (rc = S->cuda(cudaMemcpy(&mb, (void*)gp, sizeof mb, cudaMemcpyDeviceToHost), "model size")))
+        (rc = S->cuda(cudaMemcpy(&mb, (void*)gp, sizeof mb, cudaMemcpyDeviceToHost), "model size")) ||
+        (rc = S->drvcall(S->drv->moduleGetGlobal(&gp, &gb, S->mod_set, "lg_set_shape"), "set shape")) ||
+        (rc = S->cuda(cudaMemcpy(S->set_shape, (void*)gp, sizeof S->set_shape, cudaMemcpyDeviceToHost), "set shape")))
         return rc;
     S->model_bytes = mb;
 
@@ -416,7 +421,7 @@ int enqueue_systems(lg_systems* S, cudaEvent_t* ev)
     int total = S->max_total;
     void* a_setp[] = {&S->d_params, &total, &S->d_models};
     if ((rc = mark(0)) ||
-        (rc = S->launch(S->f_setp, dim3((total + 127) / 128), dim3(128), 0, a_setp, "set_params")) ||
+        (rc = S->launch(S->f_setp, dim3((total + S->set_shape[0] - 1) / S->set_shape[0]), dim3(S->set_shape[1]), 0, a_setp, "set_params")) ||
         (rc = mark(1)))
         return rc;
     if (S->psf) {

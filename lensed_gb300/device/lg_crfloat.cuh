@@ -28,7 +28,8 @@
 // for the CPU tests) or float2 (two rays, with the paired f32x2
 // instructions); the full phases take one value at a time.  Every operation
 // is a single IEEE round-to-nearest operation (no contraction is left to the
-// compiler).  Tables: lg_crf_tables.cuh, generated by make_crf_tables.py.
+// compiler).  Tables: lg_crf_tables.cuh and lg_crf_consts.cuh, generated by
+// make_crf_tables.py.
 
 #ifdef LG_CRF_HOST
 #include <cmath>
@@ -253,10 +254,25 @@ LG_CRF_DEV float2 crf_abs(float2 a)
     return v;
 }
 
-// (the library embeds the tables here for NVRTC, which has no include path)
-#ifndef LG_CRF_TABLES_INLINE
-#include "lg_crf_tables.cuh"
+// (the library embeds the constants here for NVRTC, which has no include path)
+#ifndef LG_CRF_CONSTS_INLINE
+#include "lg_crf_consts.cuh"
 #endif
+// The tables: the array itself, or in NVRTC modules (LG_CRF_MODULE) a pointer
+// to the library's copy on the device, which the host stores after loading
+// the module.
+#ifdef LG_CRF_MODULE
+extern "C" __device__ const unsigned long long* lg_crf_base;
+__device__ const unsigned long long* lg_crf_base;
+#define LG_CRF_WORDS lg_crf_base
+#else
+#include "lg_crf_tables.cuh"
+#define LG_CRF_WORDS lg_crf_words
+#endif
+#define lg_crf_exp_tab (LG_CRF_WORDS + LG_CRF_AT_EXP)
+#define lg_crf_log_tab (LG_CRF_WORDS + LG_CRF_AT_LOG)
+#define lg_crf_sc_tab (LG_CRF_WORDS + LG_CRF_AT_SC)
+#define lg_crf_q_tab (LG_CRF_WORDS + LG_CRF_AT_Q)
 
 // Entry of a quick-phase table: base (LG_CRF_Q_*) plus a byte offset.  With
 // LG_CRF_SMEM the tables (24.6 KB) are read from a copy in shared memory that
@@ -602,6 +618,7 @@ LG_CRF_DEV float crf_full_atanh(float v)
     return a < 1.0f && z1 == z2 ? crf_copysignf(z1, v) : crf_slow_atanh(v);
 }
 
+#ifndef LG_CRF_NO_QUICK
 // ------------------------------------------------------------ quick phases --
 // exp, log, atan and atanh as the exact render calls them: a first phase of
 // 16-24 operations whose error is far below half a float ulp, Ziv's test on
@@ -618,12 +635,7 @@ LG_CRF_DEV float2 crf_mulx(float2 a, float2 b) { return __fmul2_rn(a, b); }
 #ifndef LG_CRF_REST_COUNT
 #define LG_CRF_REST_COUNT()
 #endif
-LG_CRF_COLD float crf_rest_exp(float x)
-{
-    LG_CRF_REST_COUNT();
-    if (x <= LG_CRF_EXP_ZERO) return 0.0f;  // the wings of compact profiles
-    return crf_full_exp(x);
-}
+LG_CRF_COLD float crf_rest_exp(float x) { LG_CRF_REST_COUNT(); return x <= LG_CRF_EXP_ZERO ? 0.0f : crf_full_exp(x); }
 LG_CRF_COLD float crf_rest_log(float x) { LG_CRF_REST_COUNT(); return crf_full_log(x); }
 LG_CRF_COLD float crf_rest_atan(float x) { LG_CRF_REST_COUNT(); return crf_full_atan(x); }
 LG_CRF_COLD float crf_rest_atanh(float x) { LG_CRF_REST_COUNT(); return crf_full_atanh(x); }
@@ -689,6 +701,10 @@ LG_CRF_DEV F lg_crf_exp(F x)
         crf_set(out, i, crf_from_bits(crf_qexp_scale(crf_bits(crf_get(z1, i)), crf_bits(crf_get(big, i)))));
     }
     if (!crf_all<F>(ok)) {
+        bool zero[2];  // the wings of compact profiles
+#pragma unroll
+        for (int i = 0; i < crf_lanes<F>::n; ++i) zero[i] = crf_get(x, i) <= LG_CRF_EXP_ZERO;
+        if (crf_all<F>(zero)) return crf_bc<F>(0.0f);
 #pragma unroll
         for (int i = 0; i < crf_lanes<F>::n; ++i)
             if (!ok[i]) crf_set(out, i, crf_rest_exp(crf_get(x, i)));
@@ -899,6 +915,7 @@ LG_CRF_DEV F lg_crf_atanh(F v)
     }
     return out;
 }
+#endif  // LG_CRF_NO_QUICK
 
 // ------------------------------------------------- sincos, pow, atan2 (scalar) --
 // The EPL lens's functions, one value at a time (the exact render calls the
@@ -1073,6 +1090,7 @@ LG_CRF_DEV float lg_crf_atan2(float y, float x)
     return crf_slow_atan2(y, x);
 }
 
+#ifndef LG_CRF_NO_QUICK
 // ------------------------------------------- quick phases of the EPL lens --
 // x^y for one exponent: ln x = s1 + a from the quick log (a its float part,
 // absolute error 1.375 2^-34 with its rounding), t = y ln x as a double word
@@ -1238,3 +1256,4 @@ LG_CRF_DEV void crf_quick_polar(F X, F Y, F& r, F& c, F& s, F& c2, F& s2, bool (
     }
     s2 = crf_add(s2, s2);
 }
+#endif  // LG_CRF_NO_QUICK

@@ -27,3 +27,40 @@
 #define cbrtf(x) lg_cr_cbrtf(x)
 #define erff(x) lg_cr_erff(x)
 #define erfcf(x) lg_cr_erfcf(x)
+
+#ifdef LG_CRF_NO_QUICK
+// The set_params module: the functions that lg_crfloat.cuh evaluates in
+// single-precision arithmetic give the same values (the double evaluation
+// rounded once) without GB300's slow FP64 -- one candidate's Sersic object
+// took 8 us in it, most of it in four logarithms, a sine and a cosine.
+LG_DEV float lg_set_sinf(float x)
+{
+    float s, c;
+    lg_crf_sincos(x, &s, &c);
+    return s;
+}
+LG_DEV float lg_set_cosf(float x)
+{
+    float s, c;
+    lg_crf_sincos(x, &s, &c);
+    return c;
+}
+#undef expf
+#undef logf
+#undef powf
+#undef sinf
+#undef cosf
+#undef sincosf
+#undef atanf
+#undef atan2f
+#undef atanhf
+#define expf(x) crf_full_exp(x)
+#define logf(x) crf_full_log(x)
+#define powf(x, y) lg_crf_pow(x, y)
+#define sinf(x) lg_set_sinf(x)
+#define cosf(x) lg_set_cosf(x)
+#define sincosf(x, s, c) lg_crf_sincos(x, s, c)
+#define atanf(x) crf_full_atan(x)
+#define atan2f(y, x) lg_crf_atan2(y, x)
+#define atanhf(x) crf_full_atanh(x)
+#endif

@@ -1,11 +1,12 @@
-"""Generate lg_crf_tables.cuh: the tables and split constants of the
-correctly rounded single-precision functions in lg_crfloat.cuh.
+"""Generate lg_crf_tables.cuh, the tables, and lg_crf_consts.cuh, their
+offsets and the split constants, of the correctly rounded single-precision
+functions in lg_crfloat.cuh.
 
 Every value is computed with mpmath at 60 significant digits and rounded to
 float (round to nearest even) once; a "double-word" pair (hi, lo) holds
-hi = RN(v) and lo = RN(v - hi).  The tables are written as 64-bit words, two
-floats each: NVRTC reads them with every model it compiles, and one integer
-literal takes it a third of the time of a braced pair of float literals.
+hi = RN(v) and lo = RN(v - hi).  All tables are one array of 64-bit words, two
+floats each; the library holds it on the device and NVRTC modules reach it
+through a pointer, so that no model's compilation has to read them.
 
   exp   T_j = 2^(j/64), j = 0..63, as (hi, lo)                (Tang 1989);
         for the quick phase 2^(j/1024), j = 0..1023, as (hi, lo + D) with D
@@ -67,14 +68,14 @@ def word(*fs) -> str:
 
 
 def main():
-    out = ["// generated by lensed_gb300/device/make_crf_tables.py -- do not edit",
-           "// Tables of the correctly rounded single-precision functions (lg_crfloat.cuh).", ""]
+    head = "// generated by lensed_gb300/device/make_crf_tables.py -- do not edit"
+    tabs = {}
     # exp: 2^(j/64)
     rows = []
     for j in range(64):
         hi, lo = split(mp.power(2, mp.mpf(j) / 64))
         rows.append(word(hi, lo))
-    out.append("LG_CRF_TABLE(lg_crf_exp_tab, 64) = {\n    " + ",\n    ".join(rows) + "};")
+    tabs["EXP"] = rows
     # log: (c, -ln c hi, -ln c lo, 0)
     rows = []
     for j in range(1024):
@@ -85,7 +86,7 @@ def main():
         c = 1.0 if j in (511, 512) else rn(1 / (m0 + w / 2))
         hi, lo = split(-mp.log(mp.mpf(c)))
         rows.append(word(c, hi, lo, 0.0))
-    out.append("LG_CRF_TABLE(lg_crf_log_tab, 2 * 1024) = {\n    " + ",\n    ".join(rows) + "};")
+    tabs["LOG"] = rows
     # exp, quick phase: 2^(j/1024) as (hi, lo + D)
     D = mp.mpf(float.fromhex("0x1.ap-35"))
     rows = []
@@ -116,15 +117,6 @@ def main():
         rows.append(word(hi, lo))
     rows += [word(0.0, 0.0)] * 50
     quick["ATANH"] = rows
-    # the tables of the quick phases in one array, copied to shared memory as a
-    # whole; LG_CRF_Q_*: first entry of each
-    allrows = []
-    for name, r in quick.items():
-        out.append(f"#define LG_CRF_Q_{name} {len(allrows)}")
-        allrows += r
-    allrows += [word(0.0, 0.0)] * (len(allrows) % 2)
-    out.append(f"#define LG_CRF_Q_ENTRIES {len(allrows)}")
-    out.append(f"LG_CRF_TABLE(lg_crf_q_tab, {len(allrows)}) = {{\n    " + ",\n    ".join(allrows) + "};")
     # sin / cos(j/256), j = -201..201, as (sin hi, sin lo, cos hi, cos lo)
     rows = []
     for j in range(-201, 202):
@@ -132,7 +124,21 @@ def main():
         sh, sl = split(mp.sin(a))
         ch, cl = split(mp.cos(a))
         rows.append(word(sh, sl, ch, cl))
-    out.append("LG_CRF_TABLE(lg_crf_sc_tab, 2 * 403) = {\n    " + ",\n    ".join(rows) + "};")
+    tabs["SC"] = rows
+    # first word of each table; those of the quick phases side by side, as
+    # they are copied to shared memory (LG_CRF_Q_*: relative to LG_CRF_AT_Q)
+    words, defs, q = [], [], 0
+    for name in ("EXP", "LOG", "SC"):
+        defs.append(f"#define LG_CRF_AT_{name} {len(words)}")
+        words += [w.strip() for r in tabs[name] for w in r.split(",")]
+        words += [word(0.0, 0.0)] * (len(words) % 2)
+    defs.append(f"#define LG_CRF_AT_Q {len(words)}")
+    for name in ("EXP", "LOG", "ATAN", "ATANH"):
+        defs.append(f"#define LG_CRF_Q_{name} {q}")
+        words += quick[name]
+        q += len(quick[name])
+    words += [word(0.0, 0.0)] * (q % 2)
+    defs.append(f"#define LG_CRF_Q_ENTRIES {q + q % 2}")
     # split constants
     consts = {}
     l64 = mp.log(2) / 64
@@ -160,12 +166,12 @@ def main():
     if mp.mpf(f) > t:  # e^f > 2^-150: step one float down (away from zero)
         f = struct.unpack("f", struct.pack("I", struct.unpack("I", struct.pack("f", f))[0] + 1))[0]
     consts["LG_CRF_EXP_ZERO"] = f
-    for k, v in consts.items():
-        out.append(f"#define {k} ({lit(v)})")
-    text = "\n".join(out) + "\n"
-    with open(os.path.join(HERE, "lg_crf_tables.cuh"), "w") as fh:
-        fh.write(text)
-    print(f"wrote {len(text)} bytes")
+    defs += [f"#define {k} ({lit(v)})" for k, v in consts.items()]
+    for name, lines in (("consts", ["// Table offsets and split constants of the correctly rounded functions."] + defs),
+                        ("tables", ["// Tables of the correctly rounded functions (lg_crfloat.cuh).",
+                                    f"LG_CRF_TABLE(lg_crf_words, {len(words)}) = {{\n    " + ",\n    ".join(words) + "};"])):
+        with open(os.path.join(HERE, f"lg_crf_{name}.cuh"), "w") as fh:
+            fh.write("\n".join([head] + lines) + "\n")
 
 
 if __name__ == "__main__":
