@@ -71,28 +71,34 @@ void emit_compute(std::ostringstream& o, const Model& m)
 // with the pair; any other plugin is called once per ray.
 void emit_compute2(std::ostringstream& o, const Model& m)
 {
+    // (the first deflection of a plane and the first brightness are not added
+    // to a zero: the sum differs at most in the sign of a zero)
     o << "#define LG_PAIRED 1\n";
     o << "LG_DEV lg_pair lg_compute2(const lg_model& m, lg_pair2 x)\n{\n"
       << "    lg_pair2 y = x;\n    lg_pair f = lg_pair_of(0.0f);\n"
       << "    lg_pair2 a = {lg_pair_of(0.0f), lg_pair_of(0.0f)};\n";
     int trigger = 0;
+    bool first_a = true, first_f = true;
     for (size_t i = 0; i < m.objs.size(); ++i) {
         const Plugin* p = m.objs[i].plugin;
         if (p->kind != trigger && p->kind != LG_FOREGROUND) {
-            if (trigger == LG_LENS) o << "    lg_deflect(y, a);\n    a = {lg_pair_of(0.0f), lg_pair_of(0.0f)};\n";
+            if (trigger == LG_LENS) o << "    lg_deflect(y, a);\n";
             trigger = p->kind;
+            first_a = true;
         }
         const char* fn = p->kind == LG_LENS ? "lg_deflection_" : (p->kind == LG_SOURCE ? "lg_brightness_" : "lg_foreground_");
-        const char* acc = p->kind == LG_LENS ? "a" : "f";
+        bool& first = p->kind == LG_LENS ? first_a : first_f;
+        const char* acc = p->kind == LG_LENS ? (first ? "a =" : "a +=") : (first ? "f =" : "f +=");
+        first = false;
         const char* arg = p->kind == LG_FOREGROUND ? "x" : "y";
         const std::string obj = "&m.o" + std::to_string(i);
         if (p->paired) {
-            o << "    " << acc << " += " << fn << p->name << "(" << obj << ", " << arg << ");\n";
+            o << "    " << acc << " " << fn << p->name << "(" << obj << ", " << arg << ");\n";
         } else if (p->kind == LG_LENS) {
-            o << "    a += lg_pair2_join(" << fn << p->name << "(" << obj << ", lg_lane(y, 0)), " << fn << p->name
-              << "(" << obj << ", lg_lane(y, 1)));\n";
+            o << "    " << acc << " lg_pair2_join(" << fn << p->name << "(" << obj << ", lg_lane(y, 0)), " << fn
+              << p->name << "(" << obj << ", lg_lane(y, 1)));\n";
         } else {
-            o << "    f += lg_pair_of(" << fn << p->name << "(" << obj << ", lg_lane(" << arg << ", 0)), " << fn
+            o << "    " << acc << " lg_pair_of(" << fn << p->name << "(" << obj << ", lg_lane(" << arg << ", 0)), " << fn
               << p->name << "(" << obj << ", lg_lane(" << arg << ", 1)));\n";
         }
     }
@@ -189,10 +195,10 @@ void emit_prelude(std::ostringstream& o, Fp mode, bool set, const Shape& s)
 }  // namespace
 
 // The exact modules keep the tables of the correctly rounded functions
-// (24.6 KB) in shared memory, unless the values a quadrature split gathers
+// (28.7 KB) in shared memory, unless the values a quadrature split gathers
 // there (one point of each thread at least) leave too little of the 48 KB a
 // block may declare.
-bool crf_in_smem(const Shape& s, Fp mode) { return mode == Fp::EXACT && (s.qs == 1 || 4 * s.rt * s.rppt <= 22 * 1024); }
+bool crf_in_smem(const Shape& s, Fp mode) { return mode == Fp::EXACT && (s.qs == 1 || 4 * s.rt * s.rppt <= 18 * 1024); }
 
 std::string compose_source(const Model& m, const Shape& s, Fp mode, Part part)
 {

@@ -297,9 +297,7 @@ int create_systems(lg_systems* S, const lg_image_desc* images, int nsys, const l
     // and partial sums depend on the launch shape (apply_shape)
     const lg::Fp mode = lg::fp_mode(S->flags);
     // exact mode with PSFs: 256 render threads share one copy of the function
-    // tables (512 pixels a unit: 9.46 -> 9.28 ms on six systems of 64 to 512
-    // pixels a side); without PSFs the unit sets the grouping of the chi^2
-    // sums, which stays the single contexts'
+    // tables, as in the single contexts
     if (mode == lg::Fp::EXACT && S->psf) S->shape.rt = 256;
     long long img = 0, raw = 0;
     int psf_off = 0;

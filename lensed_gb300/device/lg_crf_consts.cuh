@@ -7,8 +7,8 @@
 #define LG_CRF_Q_EXP 0
 #define LG_CRF_Q_LOG 1024
 #define LG_CRF_Q_ATAN 2050
-#define LG_CRF_Q_ATANH 2563
-#define LG_CRF_Q_ENTRIES 3076
+#define LG_CRF_Q_ATANH 3075
+#define LG_CRF_Q_ENTRIES 3588
 #define LG_CRF_EXP_INVL (0x1.715476p+6f)
 #define LG_CRF_EXP_LHI (0x1.62e43p-7f)
 #define LG_CRF_EXP_LLO (-0x1.05c61p-35f)

@@ -275,7 +275,7 @@ __device__ const unsigned long long* lg_crf_base;
 #define lg_crf_q_tab (LG_CRF_WORDS + LG_CRF_AT_Q)
 
 // Entry of a quick-phase table: base (LG_CRF_Q_*) plus a byte offset.  With
-// LG_CRF_SMEM the tables (24.6 KB) are read from a copy in shared memory that
+// LG_CRF_SMEM the tables (28.7 KB) are read from a copy in shared memory that
 // the kernel fills with crf_load_tables first: a lookup is then two or three
 // instructions (32-bit offsets, the table's address an immediate) instead of
 // the five of a global load with its 64-bit address, and the table reads are
@@ -643,13 +643,13 @@ LG_CRF_COLD float crf_rest_atanh(float x) { LG_CRF_REST_COUNT(); return crf_full
 // integer fields, in inline PTX as above:
 //   exp: z 2^m for k = 1024 m + j, big's bits = bits(1.5 2^23) + k (the
 //        constant's bits leave the word in the shift)
-//   log: the mantissa in [1, 2) and the biased exponent times 2^23
+//   log: the mantissa in [1, 2) and the sign and biased exponent (times 2^23)
 #ifdef LG_CRF_HOST
 LG_CRF_DEV int crf_qexp_scale(int zbits, int bits) { return (int)((unsigned)zbits + ((unsigned)(bits & ~1023) << 13)); }
 LG_CRF_DEV void crf_qlog_fields(int b, int& mb, int& te)
 {
     mb = (b & 0x007fffff) | 0x3f800000;
-    te = b & 0x7f800000;
+    te = b & (int)0xff800000;
 }
 #else
 LG_CRF_DEV int crf_qexp_scale(int zbits, int bits)
@@ -662,23 +662,27 @@ LG_CRF_DEV int crf_qexp_scale(int zbits, int bits)
 }
 LG_CRF_DEV void crf_qlog_fields(int b, int& mb, int& te)
 {
-    asm("{\n.reg .b32 t;\nand.b32 t, %2, 0x007fffff;\nor.b32 %0, t, 0x3f800000;\nand.b32 %1, %2, 0x7f800000;\n}"
+    asm("{\n.reg .b32 t;\nand.b32 t, %2, 0x007fffff;\nor.b32 %0, t, 0x3f800000;\nand.b32 %1, %2, 0xff800000;\n}"
         : "=r"(mb), "=r"(te)
         : "r"(b));
 }
 #endif
 
-// e^x, |x| <= 87: x = k ln2/1024 + r, |r| <= 2^-11.5, k = 1024 m + j; with
-// T = 2^(j/1024) = th + tl, e^x 2^-m = th + (th rh + (th (rl + rh (rh/2 + rl)) + tl
+#define LG_CRF_QEXP_REM (0x1.ap-34f - 0x1p-24f)
+// e^x, |x| <= 87: x = k ln2/1024 + r, |r| <= 2^-11.5, k - 1 = 1024 m + j; with
+// T = 2^((j + 1)/1024) = th + tl in (1, 2], e^x 2^-m = th + (th rh + (th (rl + rh (rh/2 + rl)) + tl
 // + tl rh)): rh = x - k L_hi exact, rl = -k L_lo.  Absolute error of the sum before its
 // rounding: that of the inner sum (2^-35), r^3/6 (2^-36.2 with T < 2), the
 // rest below 2^-41; the table's second entry holds tl + D with D = 1.625
-// 2^-35, the interval's half-width.
+// 2^-35, the interval's half-width, so z = th + c rounds its upper end.  th +
+// c - 2D rounds to z too if the exact remainder of that sum, c - (z - th), is at
+// least 2D - 2^-24: z is above 1 (why k - 1), so half an ulp below it is 2^-24
+// at least.
 template <class F>
 LG_CRF_DEV F lg_crf_exp(F x)
 {
-    const F big = crf_fma(x, crf_bc<F>(LG_CRF_QEXP_INVL), crf_bc<F>(0x1.8p23f));
-    const F kf = crf_add(big, crf_bc<F>(-0x1.8p23f));
+    const F big = crf_fma(x, crf_bc<F>(LG_CRF_QEXP_INVL), crf_bc<F>(0x1.7ffffep23f));
+    const F kf = crf_add(big, crf_bc<F>(-0x1.7ffffep23f));
     const F rh = crf_fma(kf, crf_bc<F>(-LG_CRF_QEXP_LHI), x);
     const F rl = crf_mulx(kf, crf_bc<F>(-LG_CRF_QEXP_LLO));
     const F sm = crf_fma(rh, crf_fma(rh, crf_bc<F>(0.5f), rl), rl);
@@ -689,16 +693,15 @@ LG_CRF_DEV F lg_crf_exp(F x)
         crf_set(th, i, T.x);
         crf_set(tl, i, T.y);
     }
-    const F w1 = crf_fma(th, sm, crf_fma(tl, rh, tl));
-    const F w2 = crf_add(w1, crf_bc<F>(-0x1.ap-34f));
-    const F z1 = crf_add(th, crf_fma(th, rh, w1));
-    const F z2 = crf_add(th, crf_fma(th, rh, w2));
+    const F c = crf_fma(th, rh, crf_fma(th, sm, crf_fma(tl, rh, tl)));
+    const F z = crf_add(th, c);
+    const F rem = crf_sub(c, crf_sub(z, th));
     F out;
     bool ok[2];
 #pragma unroll
     for (int i = 0; i < crf_lanes<F>::n; ++i) {
-        ok[i] = crf_fabsf(crf_get(x, i)) <= 87.0f && crf_get(z1, i) == crf_get(z2, i);
-        crf_set(out, i, crf_from_bits(crf_qexp_scale(crf_bits(crf_get(z1, i)), crf_bits(crf_get(big, i)))));
+        ok[i] = crf_fabsf(crf_get(x, i)) <= 87.0f && crf_get(rem, i) >= LG_CRF_QEXP_REM;
+        crf_set(out, i, crf_from_bits(crf_qexp_scale(crf_bits(crf_get(z, i)), crf_bits(crf_get(big, i)))));
     }
     if (!crf_all<F>(ok)) {
         bool zero[2];  // the wings of compact profiles
@@ -712,16 +715,19 @@ LG_CRF_DEV F lg_crf_exp(F x)
     return out;
 }
 
-// ln x, x normal: x = 2^e m, m in [1, 2), c = 1/m cut to 11 significant bits
-// (from the reciprocal estimate; any estimate serves), so that r = m c - 1
-// (|r| <= 2^-10) is exact; ln x = (e ln2_hi + Lh) + (r + (r^2 (r/3 - 1/2) + e
-// ln2_lo + Ll)) with -ln c = Lh + Ll, Lh and ln2_hi multiples of 2^-17: the
-// first sum is exact.  Absolute error: the sum with r (2^-34 at most, the
-// rest of it reaching 2^-11), e ln2_lo + Ll (2^-36), r^4/4 (2^-42); D =
-// 1.375 2^-34.  Results near 0 are left to the full phase.
-// Out: s1, r and t with ln x = s1 + (r + t).
+// ln x, 2^-90 <= x < 2^91: x = 2^e m, m in [1, 2), c = 1/m cut to 11
+// significant bits (from the reciprocal estimate; any estimate serves), so that
+// r = m c - 1 (|r| <= 2^-10) is exact; ln x = ((e - 1/2) ln2_hi + Lh) + (r + (r^2
+// (r/3 - 1/2) + (e - 1/2) ln2_lo + Ll)) with ln2/2 - ln c = Lh + Ll, ln2_hi a
+// multiple of 2^-17 and Lh of 2^-18: the first sum is exact.  (The half centres
+// the exponents that one comparison of |e - 1/2| then admits; zero, subnormal,
+// negative, infinite and NaN x fail it.)  Absolute error: the sum with r (2^-34
+// at most), (e - 1/2) ln2_lo + Ll (2^-36), r^4/4 (2^-42); the table's Ll holds
+// D = 1.375 2^-34 more, and the interval's lower end is 3.75 2^-34 below, its
+// own rounding included.  Results near 0 are left to the full phase.
+// Out: s1, r and t with ln x + D = s1 + (r + t), and e - 1/2 (times 2^23).
 template <class F>
-LG_CRF_DEV void crf_quick_log(F x, F& s1, F& r, F& t)
+LG_CRF_DEV void crf_quick_log(F x, F& s1, F& r, F& t, F& e)
 {
     F m, c, Lh, Ll, ef;
 #pragma unroll
@@ -737,24 +743,25 @@ LG_CRF_DEV void crf_quick_log(F x, F& s1, F& r, F& t)
         crf_set(ef, i, (float)te);  // exact
     }
     r = crf_fma(m, c, crf_bc<F>(-1.0f));
-    const F e = crf_add(ef, crf_bc<F>(-127.0f * 0x1p23f));
+    e = crf_add(ef, crf_bc<F>(-127.5f * 0x1p23f));
     s1 = crf_fma(e, crf_bc<F>(LG_CRF_QLN2_HI), Lh);
     const F lo = crf_fma(e, crf_bc<F>(LG_CRF_QLN2_LO), Ll);
     const F w = crf_fma(r, crf_bc<F>(0x1.555556p-2f), crf_bc<F>(-0.5f));
     t = crf_fma(crf_mulx(r, r), w, lo);
 }
+#define LG_CRF_QLOG_E (90.5f * 0x1p23f)
 template <class F>
 LG_CRF_DEV F lg_crf_log(F x)
 {
-    F s1, r, t;
-    crf_quick_log(x, s1, r, t);
-    const F z1 = crf_add(s1, crf_add(r, crf_add(t, crf_bc<F>(0x1.6p-34f))));
-    const F z2 = crf_add(s1, crf_add(r, crf_add(t, crf_bc<F>(-0x1.6p-34f))));
-    F out = z1;
+    F s1, r, t, e;
+    crf_quick_log(x, s1, r, t, e);
+    const F a = crf_add(r, t);
+    F out = crf_add(s1, a);
+    const F z2 = crf_add(s1, crf_add(a, crf_bc<F>(-0x1.ep-33f)));
     bool ok[2];
 #pragma unroll
     for (int i = 0; i < crf_lanes<F>::n; ++i)
-        ok[i] = (unsigned)crf_bits(crf_get(x, i)) - 0x00800000u < 0x7f000000u && crf_get(z1, i) == crf_get(z2, i);
+        ok[i] = crf_fabsf(crf_get(e, i)) <= LG_CRF_QLOG_E && crf_get(out, i) == crf_get(z2, i);
     if (!crf_all<F>(ok)) {
 #pragma unroll
         for (int i = 0; i < crf_lanes<F>::n; ++i)
@@ -771,7 +778,7 @@ LG_CRF_DEV void crf_quick_ziv(F hi, F lo, F& z1, F& z2)
     z2 = crf_add(hi, crf_fma(hi, crf_bc<F>(-0x1p-38f), lo));
 }
 
-// atan t for t in [0, 1] (callers keep every t, NaN included, in that range:
+// atan t for t in [0, 2] (callers keep every t, NaN included, in that range:
 // it indexes the table): with t_j = j/512 nearest t, n = t - t_j and d = n /
 // (1 + t_j^2) (the denominator exact), atan t = atan t_j + d - t_j d^2 + (t_j^2
 // - 1/3) d^3 + O(d^4 t_j) (Taylor's series in d; |d| <= 2^-10, the omitted
@@ -807,7 +814,7 @@ LG_CRF_DEV void crf_quick_atan(F t, F tl, F& s1, F& lo)
     const F ne = crf_add(nd, crf_fma(Ah, crf_bc<F>(-1.0f), s1));
     lo = crf_fma(crf_add(ne, nc), crf_bc<F>(-1.0f), Al);
 }
-// pairs with a lane above 1 (or NaN): t = 1/a there as a double word (a >
+// pairs with a lane above 2 (or NaN): t = 1/a in lanes above 1 as a double word (a >
 // 2^126 flushes it to 0: the result is RN(pi/2)), and pi/2 - atan t
 template <class F>
 LG_CRF_COLD F crf_wide_atan(F z)
@@ -849,7 +856,7 @@ LG_CRF_DEV F lg_crf_atan(F z)
     const F a = crf_abs(z);
     bool in = true;
 #pragma unroll
-    for (int i = 0; i < crf_lanes<F>::n; ++i) in = in && crf_get(a, i) <= 1.0f;
+    for (int i = 0; i < crf_lanes<F>::n; ++i) in = in && crf_get(a, i) <= 2.0f;  // (SIE: axis ratios from 0.45)
     if (!in) return crf_wide_atan(z);
     F s1, lo, z1, z2, out;
     crf_quick_atan<F, false>(a, a, s1, lo);
@@ -1096,23 +1103,23 @@ LG_CRF_DEV float lg_crf_atan2(float y, float x)
 // absolute error 1.375 2^-34 with its rounding), t = y ln x as a double word
 // (y s1 exactly, y a added, a two-sum; error |y| 1.875 2^-34), e^t as in
 // lg_crf_exp with the low part added to the reduction's.  The interval of
-// the exp widened by twice that error.  Positive normal x with |t| <= 86;
+// the exp widened by twice that error.  x in the log's range with |t| <= 86;
 // the rest, and undecided roundings, in the full phase.
 LG_CRF_COLD float crf_rest_pow(float x, float y) { LG_CRF_REST_COUNT(); return lg_crf_pow(x, y); }
 template <class F>
 LG_CRF_DEV F lg_crf_pow1(F x, float y)
 {
-    F s1, r, t;
-    crf_quick_log(x, s1, r, t);
-    const F a = crf_add(r, t);
+    F s1, r, t, e;
+    crf_quick_log(x, s1, r, t, e);
+    const F a = crf_add(r, crf_add(t, crf_bc<F>(-0x1.6p-34f)));
     const F Y = crf_bc<F>(y);
     const F ph = crf_mul(Y, s1);
     const F pl = crf_fma(Y, a, crf_fma(Y, s1, crf_neg(ph)));
     const F T = crf_add(ph, pl);  // two-sum
     const F bb = crf_sub(T, ph);
     const F Tl = crf_add(crf_sub(ph, crf_sub(T, bb)), crf_sub(pl, bb));
-    const F big = crf_fma(T, crf_bc<F>(LG_CRF_QEXP_INVL), crf_bc<F>(0x1.8p23f));
-    const F kf = crf_add(big, crf_bc<F>(-0x1.8p23f));
+    const F big = crf_fma(T, crf_bc<F>(LG_CRF_QEXP_INVL), crf_bc<F>(0x1.7ffffep23f));
+    const F kf = crf_add(big, crf_bc<F>(-0x1.7ffffep23f));
     const F rh = crf_fma(kf, crf_bc<F>(-LG_CRF_QEXP_LHI), T);
     const F rl = crf_fma(kf, crf_bc<F>(-LG_CRF_QEXP_LLO), Tl);
     const F sm = crf_fma(rh, crf_fma(rh, crf_bc<F>(0.5f), rl), rl);
@@ -1124,18 +1131,16 @@ LG_CRF_DEV F lg_crf_pow1(F x, float y)
         crf_set(tl, i, E.y);
     }
     const float wide = crf_mul(crf_fabsf(y), 0x1p-32f);
-    const F w0 = crf_fma(th, sm, crf_fma(tl, rh, tl));
-    const F w1 = crf_add(w0, crf_bc<F>(wide));
-    const F w2 = crf_sub(w0, crf_bc<F>(crf_add(wide, 0x1.ap-34f)));
-    const F z1 = crf_add(th, crf_fma(th, rh, w1));
-    const F z2 = crf_add(th, crf_fma(th, rh, w2));
+    const F c = crf_fma(th, rh, crf_add(crf_fma(th, sm, crf_fma(tl, rh, tl)), crf_bc<F>(wide)));
+    const F z = crf_add(th, c);
+    const F rem = crf_sub(c, crf_sub(z, th));
+    const float low = crf_fma(wide, 2.0f, LG_CRF_QEXP_REM);
     F out;
     bool ok[2];
 #pragma unroll
     for (int i = 0; i < crf_lanes<F>::n; ++i) {
-        ok[i] = (unsigned)crf_bits(crf_get(x, i)) - 0x00800000u < 0x7f000000u && crf_fabsf(crf_get(T, i)) <= 86.0f &&
-                crf_get(z1, i) == crf_get(z2, i);
-        crf_set(out, i, crf_from_bits(crf_qexp_scale(crf_bits(crf_get(z1, i)), crf_bits(crf_get(big, i)))));
+        ok[i] = crf_fabsf(crf_get(e, i)) <= LG_CRF_QLOG_E && crf_fabsf(crf_get(T, i)) <= 86.0f && crf_get(rem, i) >= low;
+        crf_set(out, i, crf_from_bits(crf_qexp_scale(crf_bits(crf_get(z, i)), crf_bits(crf_get(big, i)))));
     }
     if (!crf_all<F>(ok)) {
 #pragma unroll

@@ -429,9 +429,12 @@ LG_DEV lg_pair2 normalize(lg_pair2 a)
 LG_DEV void lg_deflect(lg_pair2& y, lg_pair2 a)
 {
     const lg_pair d = dot(a, a);
-    const float2 a0 = d.v.x < LG_INF ? lg_lane(a, 0) : make_float2(1E10f, 1E10f);
-    const float2 a1 = d.v.y < LG_INF ? lg_lane(a, 1) : make_float2(1E10f, 1E10f);
-    y -= lg_pair2_join(a0, a1);
+    if (!(d.v.x < LG_INF && d.v.y < LG_INF)) {
+        const float2 a0 = d.v.x < LG_INF ? lg_lane(a, 0) : make_float2(1E10f, 1E10f);
+        const float2 a1 = d.v.y < LG_INF ? lg_lane(a, 1) : make_float2(1E10f, 1E10f);
+        a = lg_pair2_join(a0, a1);
+    }
+    y -= a;
 }
 
 // Polar angles of a plugin's frame for two rays: r = |x|, (c, s) = (cos,

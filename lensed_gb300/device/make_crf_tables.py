@@ -9,14 +9,15 @@ floats each; the library holds it on the device and NVRTC modules reach it
 through a pointer, so that no model's compilation has to read them.
 
   exp   T_j = 2^(j/64), j = 0..63, as (hi, lo)                (Tang 1989);
-        for the quick phase 2^(j/1024), j = 0..1023, as (hi, lo + D) with D
-        the half-width of its rounding interval
+        for the quick phase 2^((j + 1)/1024), j = 0..1023, as (hi, lo + D)
+        with D the half-width of its rounding interval
   log   for the 1024 intervals of the mantissa m in [0.75, 1.5) (512 of
         width 2^-11 below 1, 512 of width 2^-10 above): c_j = RN(1 / centre)
         (c = 1 for the two intervals next to 1) and -ln(c_j) as (hi, lo)
-        (Tang 1990); for the quick phase -ln(c) of every c of 11 significant
-        bits from 1/2 - 2^-12 to 1, as (hi, lo) with hi a multiple of 2^-17
-  atan  atan(j/512), j = 0..512, as (hi, lo)
+        (Tang 1990); for the quick phase ln(2)/2 - ln(c) of every c of 11
+        significant bits from 1/2 - 2^-12 to 1, as (hi, lo + D) with hi a
+        multiple of 2^-18
+  atan  atan(j/512), j = 0..1024, as (hi, lo)
   atanh atanh(j/512), j = 0..461, as (hi, lo), padded to 512 entries
   sin/cos  sin(j/256) and cos(j/256), j = -201..201, as (hi, lo) pairs
 
@@ -87,26 +88,28 @@ def main():
         hi, lo = split(-mp.log(mp.mpf(c)))
         rows.append(word(c, hi, lo, 0.0))
     tabs["LOG"] = rows
-    # exp, quick phase: 2^(j/1024) as (hi, lo + D)
+    # exp, quick phase: 2^((j + 1)/1024) as (hi, lo + D)
     D = mp.mpf(float.fromhex("0x1.ap-35"))
     rows = []
     for j in range(1024):
-        v = mp.power(2, mp.mpf(j) / 1024)
+        v = mp.power(2, mp.mpf(j + 1) / 1024)
         hi = rn(v)
         rows.append(word(hi, rn(v - mp.mpf(hi) + D)))
     quick = {"EXP": rows}
-    # log, quick phase: -ln(c), c = float with bit pattern 0x3effe000 + j 2^13
+    # log, quick phase: ln2/2 - ln(c), c = float with bit pattern 0x3effe000 + j
+    # 2^13, as (hi, lo + D)
+    D = mp.mpf(float.fromhex("0x1.6p-34"))
     rows = []
     for j in range(1026):
         c = struct.unpack("f", struct.pack("I", 0x3EFFE000 + (j << 13)))[0]
-        v = -mp.log(mp.mpf(c))
-        hi = mp.floor(v * 2 ** 17 + mp.mpf(0.5)) / 2 ** 17
+        v = mp.log(2) / 2 - mp.log(mp.mpf(c))
+        hi = mp.floor(v * 2 ** 18 + mp.mpf(0.5)) / 2 ** 18
         assert mp.mpf(rn(hi)) == hi
-        rows.append(word(rn(hi), rn(v - hi)))
+        rows.append(word(rn(hi), rn(v - hi + D)))
     quick["LOG"] = rows
     # atan(j/512)
     rows = []
-    for j in range(513):
+    for j in range(1025):
         hi, lo = split(mp.atan(mp.mpf(j) / 512))
         rows.append(word(hi, lo))
     quick["ATAN"] = rows

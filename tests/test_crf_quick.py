@@ -46,6 +46,9 @@ WINDOWS = [
     (1, bits(2.0 ** -126) - 1000000, bits(2.0 ** -126) + 1000000),  # log: the smallest normal
     (1, bits(3.4e38), bits(float("inf")) + 1000),                  # log: the largest, infinite, NaN
     (2, bits(0.999), bits(1.001)), (2, bits(9e-4), bits(3e-3)),    # atan: both sides of 1; the first entries
+    (2, bits(1.999), bits(2.001)),                                 # atan: the end of the table
+    (1, bits(2.0 ** 91) - 100000, bits(2.0 ** 91) + 100000),       # log: the ends of the quick range
+    (1, bits(2.0 ** -90) - 100000, bits(2.0 ** -90) + 100000),
     (2, bits(8e37), bits(float("inf")) + 1000),                    # atan: 1/a flushed to 0, infinite, NaN
     (3, bits(0.899), bits(0.901)), (3, bits(9e-4), bits(3e-3)),    # atanh: the end of the quick range; first entries
     (3, bits(0.999), bits(1.001)),                                 # atanh: 1 and above
