@@ -15,9 +15,9 @@ LG_DEV LG_SCALAR(V) lg_foreground_sky(const lg_data_sky* __restrict__ o, V x)
 {
     return o->bg + dot(o->grad, x - make_float2(1, 1));
 }
-#if defined(LG_EXACT) && !defined(LG_HOST_SET)
-// ray pairs of the exact modules: no gradient (the default) adds a zero to
-// the level at every (finite) position
+#ifndef LG_HOST_SET
+// ray pairs: no gradient (the default) adds a zero to the level at every
+// (finite) position
 LG_DEV lg_pair lg_foreground_sky(const lg_data_sky* __restrict__ o, lg_pair2 x)
 {
     if (o->grad.x == 0.0f && o->grad.y == 0.0f) return lg_pair_of(o->bg);
