@@ -76,7 +76,7 @@ extern "C" {
  *   LG_FLAG_FAST_MATH  ray pairs with FMA contraction and hardware-
  *                      approximate functions (a few ulp each; what the
  *                      reference's -cl-fast-relaxed-math build allows):
- *                      about three times the default's throughput, logL
+ *                      about twice the default's throughput, logL
  *                      within about 1e-3 + 2e-6 |logL| of the oracle's */
 #define LG_FLAG_STRICT_FP 1  /* strict mode (above) */
 #define LG_FLAG_NO_GRAPH 2   /* launch kernels directly instead of graph replay */

@@ -1,9 +1,9 @@
 // set_params on the host, for batches of a few candidates.
 //
-// One candidate's object data take 12-15 us on the GPU: the set module
-// evaluates its elementary functions in FP64 (rounded once to FP32, the
-// oracle's semantics), GB300 runs FP64 at a small fraction of its FP32 rate,
-// and one thread per object walks a dependent chain of them.  The host's
+// One candidate's object data take 6 us and more on the GPU (12-15 us where the
+// set module evaluates its elementary functions in FP64, rounded once to FP32,
+// the oracle's semantics: GB300 runs FP64 at a small fraction of its FP32 rate):
+// one thread per object walks a dependent chain of them.  The host's
 // FP64 is fast, so for a handful of candidates the object data are computed
 // here and copied to the GPU with the launch.
 //
