@@ -69,22 +69,25 @@ void emit_compute(std::ostringstream& o, const Model& m)
 // The same sum for two rays at once (lg_pair2), for the paired ray kernels
 // of the fast mode: plugins with template evaluation functions are called
 // with the pair; any other plugin is called once per ray.
-void emit_compute2(std::ostringstream& o, const Model& m)
+void emit_compute2(std::ostringstream& o, const Model& m, Fp mode)
 {
-    // (the first deflection of a plane and the first brightness are not added
-    // to a zero: the sum differs at most in the sign of a zero)
+    // (exact mode: the first deflection of a plane and the first brightness are
+    // not added to a zero, the sum differs at most in the sign of a zero; in the
+    // fast mode the addition keeps a product that ends the value from being
+    // fused into the next sum, so it stays)
     o << "#define LG_PAIRED 1\n";
     o << "LG_DEV lg_pair lg_compute2(const lg_model& m, lg_pair2 x)\n{\n"
       << "    lg_pair2 y = x;\n    lg_pair f = lg_pair_of(0.0f);\n"
       << "    lg_pair2 a = {lg_pair_of(0.0f), lg_pair_of(0.0f)};\n";
     int trigger = 0;
-    bool first_a = true, first_f = true;
+    bool first_a = mode == Fp::EXACT, first_f = first_a;
     for (size_t i = 0; i < m.objs.size(); ++i) {
         const Plugin* p = m.objs[i].plugin;
         if (p->kind != trigger && p->kind != LG_FOREGROUND) {
             if (trigger == LG_LENS) o << "    lg_deflect(y, a);\n";
+            if (trigger == LG_LENS && mode != Fp::EXACT) o << "    a = {lg_pair_of(0.0f), lg_pair_of(0.0f)};\n";
             trigger = p->kind;
-            first_a = true;
+            first_a = mode == Fp::EXACT;
         }
         const char* fn = p->kind == LG_LENS ? "lg_deflection_" : (p->kind == LG_SOURCE ? "lg_brightness_" : "lg_foreground_");
         bool& first = p->kind == LG_LENS ? first_a : first_f;
@@ -265,7 +268,7 @@ std::string compose_source(const Model& m, const Shape& s, Fp mode, Part part)
         o << "#define LG_HAS_PSF 0\n";
     }
     emit_compute(o, m);
-    if (!strict) emit_compute2(o, m);
+    if (!strict) emit_compute2(o, m, mode);
     o << kernels_source() << "\n";
     return o.str();
 }
@@ -299,7 +302,7 @@ std::string compose_multi_source(const Model& m, const std::vector<std::pair<int
         o << (n ? ", " : "") << "{" << hexf((float)m.rule->weig[n]) << ", " << hexf((float)m.rule->errw[n]) << "}";
     o << "};\n";
     emit_compute(o, m);
-    if (!strict) emit_compute2(o, m);
+    if (!strict) emit_compute2(o, m, mode);
     o << "#define LG_PSF_SHAPES";
     for (const auto& ps : psf_shapes) o << " LG_PSF_CASE(" << ps.first << ", " << ps.second << ")";
     o << "\n";
