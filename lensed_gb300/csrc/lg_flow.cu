@@ -191,6 +191,10 @@ __device__ void dense_fwd_tile(const float* X, int ldx, int K, const float* Ws, 
             for (int j = 0; j < CPT; ++j) acc[i][j] = 0.0f;
         int k = 0;
         if (vec)
+// two warps a scheduler: the next steps' loads have to be in flight under
+// this one's products (training of 25 epochs 17.9 ms, unrolled 2 / 4 / 8
+// times 16.9 / 16.7 / 16.6)
+#pragma unroll 4
             for (; k + 3 < K; k += 4) {
                 float w[4][CPT];
 #pragma unroll
