@@ -625,9 +625,11 @@ LG_CRF_DEV float crf_full_atanh(float v)
 // its interval, and the functions above (out of line) for the lanes it
 // leaves undecided.  All F operations run on both lanes of a pair at once.
 //
-// products that enter only terms whose rounding errors the interval covers:
-// on pairs the packed multiply (contracting it into a following add would
-// only lower the error)
+// products that enter only fmas, or sums where the unrounded product serves
+// as well: on pairs the packed multiply, which the assembler may contract
+// into a following packed add.  (atanh's d, added to a table value, is such a
+// product: what its sum loses is taken against the rounded d.  atan's is not,
+// there the error term of the sum adds the product itself.)
 LG_CRF_DEV float crf_mulx(float a, float b) { return crf_mul(a, b); }
 #ifndef LG_CRF_HOST
 LG_CRF_DEV float2 crf_mulx(float2 a, float2 b) { return __fmul2_rn(a, b); }
@@ -801,7 +803,7 @@ LG_CRF_DEV void crf_quick_atan(F t, F tl, F& s1, F& lo)
     const F s = crf_fma(tj, tj, crf_bc<F>(1.0f));
 #pragma unroll
     for (int i = 0; i < crf_lanes<F>::n; ++i) crf_set(nr, i, crf_rcp(-crf_get(s, i)));
-    const F nd = crf_mulx(n, nr);
+    const F nd = crf_mul(n, nr);  // rounded: its error is in res, so ne below has to take the same value
     F res = crf_fma(nd, s, n);
     if (DW) res = crf_add(res, tl);
     F nd1 = crf_mulx(res, nr);
