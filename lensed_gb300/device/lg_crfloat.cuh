@@ -1101,12 +1101,18 @@ LG_CRF_DEV float lg_crf_atan2(float y, float x)
 
 #ifndef LG_CRF_NO_QUICK
 // ------------------------------------------- quick phases of the EPL lens --
-// x^y for one exponent: ln x = s1 + a from the quick log (a its float part,
-// absolute error 1.375 2^-34 with its rounding), t = y ln x as a double word
-// (y s1 exactly, y a added, a two-sum; error |y| 1.875 2^-34), e^t as in
-// lg_crf_exp with the low part added to the reduction's.  The interval of
-// the exp widened by twice that error.  x in the log's range with |t| <= 86;
-// the rest, and undecided roundings, in the full phase.
+// x^y for one exponent: ln x = s1 + a from the quick log (a its float part),
+// t = y ln x as a double word (y s1 exactly, y a added, a two-sum), e^t as in
+// lg_crf_exp with the low part added to the reduction's.  |a| is at most 1.135
+// 2^-10 (r, and e ln2_lo up to 2^-12.9), so in units of 2^-34: a's rounding 1,
+// those of (e - 1/2) ln2_lo + Ll, of t and of its shift back by D 1/8 each,
+// ln2_lo's own 0.09 (1.46 in all; 1.455 is met), the rounding of y a + (the
+// product's error) 1.14 |y|, and the square of t's low part, which the exp
+// leaves out, 0.125 |y| (2^-37, for |t| above 64 only, so |y| above 1).  A
+// power is below 2 times its exp's scale: 2 (1.46 + 1.14 + 0.125) |y| 2^-34 =
+// 1.36 |y| 2^-32, and the interval of the exp is widened by 1.5 |y| 2^-32 each
+// way.  x in the log's range with |t| <= 86; the rest, and undecided
+// roundings, in the full phase.
 LG_CRF_COLD float crf_rest_pow(float x, float y) { LG_CRF_REST_COUNT(); return lg_crf_pow(x, y); }
 template <class F>
 LG_CRF_DEV F lg_crf_pow1(F x, float y)
@@ -1132,7 +1138,7 @@ LG_CRF_DEV F lg_crf_pow1(F x, float y)
         crf_set(th, i, E.x);
         crf_set(tl, i, E.y);
     }
-    const float wide = crf_mul(crf_fabsf(y), 0x1p-32f);
+    const float wide = crf_mul(crf_fabsf(y), 0x1.8p-32f);
     const F c = crf_fma(th, rh, crf_add(crf_fma(th, sm, crf_fma(tl, rh, tl)), crf_bc<F>(wide)));
     const F z = crf_add(th, c);
     const F rem = crf_sub(c, crf_sub(z, th));
