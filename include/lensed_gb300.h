@@ -308,7 +308,9 @@ int lg_probe_pair_math(int device, int fn, const float* x, int n, float* out);
  * them), atan2(x, p) (7) or pow(|x|, p) (8), with p the float of bit pattern
  * u * 0x9E3779B1, one value at a time, with the function evaluated in double
  * and rounded once, for every float x whose bit pattern u lies in [lo, hi)
- * (hi <= 2^32), on a device.  *mismatches receives the number of inputs
+ * (hi <= 2^32), on a device; or, on pairs of points or bases made from u,
+ * the exact modules' paired polar frame (9: the lanes it decides) and paired
+ * power with one exponent (10).  *mismatches receives the number of inputs
  * whose results differ (NaN matches NaN); the first nfirst of their bit
  * patterns go to first. */
 int lg_probe_crf_sweep(int device, int fn, unsigned long long lo, unsigned long long hi,

@@ -5,7 +5,7 @@
 // vector of inputs, so their accuracy can be checked against
 // double-precision references on the host; and a sweep that compares the
 // correctly rounded functions with the double evaluation on the device over
-// a range of float bit patterns.
+// a range of float bit patterns, or over points and powers made from them.
 
 #include <cuda_runtime.h>
 
@@ -62,6 +62,64 @@ __device__ float crf_two_double(int fn, float x, unsigned u)
     }
 }
 
+// The EPL lens's quick phases on a pair made from u by a bit mixer: fn 9 the
+// polar frame (mismatches among its decided lanes), 10 the power with one
+// exponent.  Points of sizes 2^-33 to
+// 2^33 (a quarter of ordinary size), one in eight each near the x axis, the y
+// axis and a diagonal, others with min/max near 2^-20; bases over the whole
+// range of the quick logarithm and near 1, the lens's exponents and any up to
+// 2^8.
+__device__ unsigned long long probe_mix(unsigned long long z)
+{
+    z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
+    z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
+    return z ^ (z >> 31);
+}
+// a float of random sign and mantissa bits, of binary exponent e
+__device__ float probe_float(unsigned h, int e) { return __uint_as_float((h & 0x807fffffu) | (unsigned)(e + 127) << 23); }
+__device__ int quick_pair(int fn, unsigned u)
+{
+    float x[2], y[2];
+    unsigned h = 0;
+    for (int i = 0; i < 2; ++i) {
+        const unsigned long long z = probe_mix(2ull * u + i + 0x9E3779B97F4A7C15ull);
+        const unsigned a = (unsigned)z, b = (unsigned)(z >> 32);
+        h = (unsigned)probe_mix(z);
+        if (fn == 10) {
+            x[i] = fabsf(probe_float(a, h % 2 ? (int)(b % 181) - 90 : (int)(b % 3) - 1));
+            continue;
+        }
+        const int e = h % 4 == 0 ? 5 : (int)(h >> 8 & 63) - 31;
+        x[i] = probe_float(a, e - (h >> 14 & 1));
+        y[i] = probe_float(b, e - (h >> 15 & 1));
+        const int kind = h >> 16 & 7, small = h >> 20 & 31;
+        if (kind == 0) y[i] = probe_float(b, e - small < -120 ? -120 : e - small);
+        if (kind == 1) x[i] = probe_float(a, e - small < -120 ? -120 : e - small);
+        if (kind == 2) y[i] = (b & 1 ? x[i] : -x[i]) * (1.0f + (b >> 28) * 0x1p-23f);
+        if (kind == 3) y[i] = x[i] * 0x1p-20f * (1.0f + ((int)(b >> 28) - 8) * 0x1p-23f);
+    }
+    const float2 X = make_float2(x[0], x[1]);
+    auto same = [](float v, float w) { return __float_as_uint(v) == __float_as_uint(w) || (v != v && w != w); };
+    if (fn == 10) {
+        const float e = h & 1 ? lg_probe_y[h >> 1 & 15] : probe_float(h, (int)(h >> 23 & 15) - 7);
+        const float2 r = lg_crf_pow1(X, e);
+        return !same(r.x, (float)pow((double)x[0], (double)e)) + !same(r.y, (float)pow((double)x[1], (double)e));
+    }
+    float2 r, c, s, c2, s2;
+    bool ok[2];
+    crf_quick_polar(X, make_float2(y[0], y[1]), r, c, s, c2, s2, ok);
+    int bad = 0;
+    for (int i = 0; i < 2; ++i) {
+        if (!ok[i]) continue;
+        const float phi = (float)atan2((double)y[i], (double)x[i]);
+        const float root = __fsqrt_rn(__fadd_rn(__fmul_rn(x[i], x[i]), __fmul_rn(y[i], y[i])));
+        bad += !(same(crf_get(r, i), root) && same(crf_get(c, i), (float)cos((double)phi)) &&
+                 same(crf_get(s, i), (float)sin((double)phi)) && same(crf_get(c2, i), (float)cos((double)(2 * phi))) &&
+                 same(crf_get(s2, i), (float)sin((double)(2 * phi))));
+    }
+    return bad;
+}
+
 // every bit pattern u in [lo, hi) as lane 0 of a pair whose lane 1 is an
 // unrelated input (u times an odd constant, a bijection of the 32-bit
 // patterns), so that the lanes of a pair take different paths and table
@@ -76,6 +134,15 @@ __global__ void lg_crf_sweep_kernel(int fn, unsigned long long lo, unsigned long
     unsigned long long nbad = 0;
     for (unsigned long long u = lo + blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; u < hi; u += stride) {
         const float x0 = __uint_as_float((unsigned)u);
+        if (fn >= 9) {
+            const int n = quick_pair(fn, (unsigned)u);
+            if (n) {
+                nbad += n;
+                const unsigned long long k = atomicAdd(bad + 1, 1ull);
+                if (k < (unsigned long long)nfirst) first[k] = (unsigned)u;
+            }
+            continue;
+        }
         if (fn >= 4) {
             const float r0 = crf_two(fn, x0, (unsigned)u), w0 = crf_two_double(fn, x0, (unsigned)u);
             if (!(__float_as_uint(r0) == __float_as_uint(w0) || (r0 != r0 && w0 != w0))) {
@@ -153,7 +220,7 @@ extern "C" int lg_probe_pair_math(int device, int fn, const float* x, int n, flo
 extern "C" int lg_probe_crf_sweep(int device, int fn, unsigned long long lo, unsigned long long hi,
                                   unsigned long long* mismatches, unsigned* first, int nfirst)
 {
-    if (fn < 0 || fn > 8 || lo > hi || hi > (1ull << 32) || !mismatches || nfirst < 0 || (nfirst && !first))
+    if (fn < 0 || fn > 10 || lo > hi || hi > (1ull << 32) || !mismatches || nfirst < 0 || (nfirst && !first))
         return LG_ERR_INPUT;
     auto fail = [](cudaError_t e) {
         lg::set_global_error(cudaGetErrorString(e));

@@ -19,7 +19,9 @@
 // also what the double evaluation rounds to, its own error being far smaller
 // than the interval.  Otherwise (about one call in 2^16) the lane evaluates
 // the function in double and rounds once, exactly as the strict modules do.
-// So each function returns the double-then-round value for every input.
+// So each function returns the double-then-round value for every input (the
+// bounds are in the comments; all 2^32 inputs of the one-argument functions
+// have been compared, the others on samples).
 //
 // exp, log, atan and atanh first take a quick phase (below), whose error is
 // a few 2^-35 to 2^-39 and whose own rounding test leaves one lane in 2^9 to
@@ -927,8 +929,8 @@ LG_CRF_DEV F lg_crf_atanh(F v)
 #endif  // LG_CRF_NO_QUICK
 
 // ------------------------------------------------- sincos, pow, atan2 (scalar) --
-// The EPL lens's functions, one value at a time (the exact render calls the
-// correctly rounded functions lane by lane).
+// The EPL lens's functions, one value at a time: for scalar calls, and for
+// the lanes that the quick phases of pairs (below) leave undecided.
 
 LG_CRF_DEV void crf_two_sum(float a, float b, float& s, float& e)
 {
@@ -1164,18 +1166,36 @@ LG_CRF_DEV F lg_crf_pow1(F x, float y)
 // computation instead of an atan2 and two sincos:
 //  * H = X^2 + Y^2 as a double word (exact products; its high part is the
 //    rounded sum r is the root of), 1/sqrt(H) = y0 + y1 from the reciprocal
-//    square root estimate and one Newton step (error 2^-44), so cos and sin
-//    of the exact angle are X and Y times it;
+//    square root estimate and one Newton step, so cos and sin of the exact
+//    angle are X and Y times it;
 //  * the exact angle from the atan of min/max as in lg_crf_atan, then phi =
 //    its rounding, and rem = angle - phi;
 //  * sin phi = sin(angle) - rem cos(angle), cos phi likewise (rem^2/2 is
-//    below 2^-45), sin 2phi = 2 sin phi cos phi, cos 2phi = +-(1 - 2 m^2) with
+//    below 2^-47), sin 2phi = 2 sin phi cos phi, cos 2phi = +-(1 - 2 m^2) with
 //    m the smaller of the two.
-// The rounding tests' margins are twice the largest errors measured with
-// reciprocal estimates 2^-22 off: sin phi and sin phi cos phi 2^-38.5 |phi|
-// and 2^-40, cos phi 2^-40, cos 2phi 2^-39.  ok[i]: every rounding of lane i decided; its range
-// excludes axes and extreme sizes (min/max < 2^-20, H outside [2^-60,
-// 2^60]), which the caller sends through the one-value functions.
+// Error bounds for estimates 2^-22 off (the hardware's: 2^-23 and 2^-22.9),
+// in units of 2^-42; in brackets the largest error met on 4 10^7 points with
+// estimates that far off either way at random:
+//  * sqrt(h), relative: the square of g's error, (1.25 2^-22)^2 / 2, and the
+//    roundings of h - g^2 and of its product: 0.7 [0.6], margin 4;
+//  * 1/sqrt(H), relative: Newton's step 3/8 (2.5 2^-22)^2 = 0.6, the roundings
+//    of 1 - g y0 and of what is added to it 0.4, of y1 0.1; with the rounding
+//    of their low parts, sin and cos of the angle 1.0;
+//  * atan q, relative: q 0.5, the low part of d (up to 2.5 2^-22 of it: three
+//    roundings and the estimate) 1.1, its part in the cube, left out, 2.5, the
+//    square 0.65, the cube 0.4, the fifth power 0.8, the sums 1.5: 7.8 [4.0],
+//    near q = 2^-10; absolute 1.5 [0.6], and 2.1 with the multiple of pi/2.
+//    phi has the margin 16 |phi| of crf_quick_ziv;
+//  * sin phi: the angle's error times the cosine, the sine's 1.0 and its
+//    rounding: 9.3 |phi| [4.0] below |phi| = 0.36, margin 11 |phi|, and above
+//    2.7 [0.8], margin 4; cos phi likewise 2.7 [0.8], margin 4;
+//  * sin phi cos phi: both of these, the product of the low parts 0.5 and
+//    roundings: 12.4 |phi| [4.4] and 4.4 [0.9], margins 13.75 |phi| and 5;
+//  * cos 2phi: 4 |m| times m's error 7.2, twice the square of m's low part
+//    1.0, roundings 1.0: 9.2 [2.6], margin 10.
+// ok[i]: every rounding of lane i decided; its range excludes axes and
+// extreme sizes (min/max < 2^-20, H outside [2^-60, 2^60]), which the caller
+// sends through the one-value functions.
 template <class F>
 LG_CRF_DEV void crf_quick_polar(F X, F Y, F& r, F& c, F& s, F& c2, F& s2, bool (&ok)[2])
 {
@@ -1237,7 +1257,7 @@ LG_CRF_DEV void crf_quick_polar(F X, F Y, F& r, F& c, F& s, F& c2, F& s2, bool (
     F ms = crf_mulx(z1, crf_bc<F>(0x1.6p-39f));
 #pragma unroll
     for (int i = 0; i < crf_lanes<F>::n; ++i) crf_set(ms, i, crf_get(ms, i) < 0x1p-40f ? crf_get(ms, i) : 0x1p-40f);
-    const F mc = crf_bc<F>(0x1p-40f), mk = crf_bc<F>(0x1p-39f);
+    const F mc = crf_bc<F>(0x1p-40f), mk = crf_bc<F>(0x1.4p-39f);
     s = crf_add(sh, crf_add(sl, ms));
     const F sb = crf_add(sh, crf_sub(sl, ms));
     c = crf_add(ch, crf_add(cl, mc));
@@ -1245,8 +1265,8 @@ LG_CRF_DEV void crf_quick_polar(F X, F Y, F& r, F& c, F& s, F& c2, F& s2, bool (
     // sin 2phi
     const F ph = crf_mul(sh, ch);
     const F pl = crf_fma(sh, cl, crf_fma(sl, ch, crf_fma(sh, ch, crf_neg(ph))));
-    s2 = crf_add(ph, crf_add(pl, ms));
-    const F s2b = crf_add(ph, crf_sub(pl, ms));
+    s2 = crf_add(ph, crf_fma(ms, crf_bc<F>(1.25f), pl));
+    const F s2b = crf_add(ph, crf_fma(ms, crf_bc<F>(-1.25f), pl));
     // cos 2phi
     F mh, ml;
 #pragma unroll
