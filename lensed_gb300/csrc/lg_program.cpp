@@ -198,10 +198,20 @@ void emit_prelude(std::ostringstream& o, Fp mode, bool set, const Shape& s)
 }  // namespace
 
 // The exact modules keep the tables of the correctly rounded functions
-// (28.7 KB) in shared memory, unless the values a quadrature split gathers
-// there (one point of each thread at least) leave too little of the 48 KB a
-// block may declare.
-bool crf_in_smem(const Shape& s, Fp mode) { return mode == Fp::EXACT && (s.qs == 1 || 4 * s.rt * s.rppt <= 18 * 1024); }
+// (28.7 KB) in shared memory for blocks of 128 threads and more.  An SM has
+// room for 7 copies, so smaller blocks would leave most of its 1024 resident
+// threads out; they read the tables from global memory (the L1 holds them).
+// Render of four objects, global / shared (us): 256^2, 25 points, 256
+// candidates, 32 threads 3308 / 6797, 64 3339 / 4204, 128 3341 / 3358, 256
+// 3355 / 3197; 128^2 without a PSF, 9 points, 1024 candidates 1654 / 4213, 1435
+// / 2504, 1370 / 1550, 1341 / 1343; with three objects and 128 threads 1038 /
+// 993, and six EPL systems without a PSF 15.9 / 15.5 ms.  Nor where the values
+// a quadrature split gathers there (one point of each thread at least) leave
+// too little of the 48 KB a block may declare.
+bool crf_in_smem(const Shape& s, Fp mode)
+{
+    return mode == Fp::EXACT && s.rt >= 128 && (s.qs == 1 || 4 * s.rt * s.rppt <= 18 * 1024);
+}
 
 std::string compose_source(const Model& m, const Shape& s, Fp mode, Part part)
 {
