@@ -118,7 +118,18 @@ typedef struct {
 typedef struct {
     const char* rule; /* quadrature rule name, NULL = "g3k7" (src/input/options.c:130-135) */
     int device;       /* CUDA device ordinal */
-    int max_batch;    /* largest B per call (scratch sizing); 0 = 1024 */
+    int max_batch;    /* largest B per call; 0 = 1024.  It sizes the scratch and
+                       * chooses the kernels: a context whose largest batch is
+                       * one or a few candidates is compiled with its
+                       * convolution tiles split over clusters of blocks and,
+                       * in the exact mode, its quadrature over 2 or 4 threads
+                       * (lg_split_tiles), which a context made for more does
+                       * not use for a small B either.  The values are the
+                       * same.  So a host sampler that asks for one point at a
+                       * time is served faster by a context of its own with
+                       * max_batch = 1; its program is another one than a batch
+                       * context's of the same model, and the first of each in
+                       * a process is compiled (about half a second). */
     int flags;        /* LG_FLAG_* */
 } lg_options;
 
@@ -160,7 +171,9 @@ long lg_make_weight(const float* image, long n, const float* weight_map, const f
                     double offset, const float* xweight, const int* mask, float* weight_out);
 
 /* Compose and compile the program for a model without creating a context or
- * touching a GPU (configuration check; usable on machines without a GPU). */
+ * touching a GPU (configuration check; usable on machines without a GPU):
+ * that of a context for opts->max_batch candidates, 0 or no opts meaning
+ * many. */
 int lg_compile_check(const lg_image_desc* image, const lg_object_desc* objs, int nobjs, const lg_options* opts,
                      char* log, size_t log_size);
 
@@ -273,7 +286,13 @@ int lg_eval_profile(lg_ctx* ctx, const double* d_params, int B, double* d_logL, 
  * are the same for every shape up to the order of FP64 partial sums, and,
  * with a quadrature split above 1, of the FP32 quadrature sum. */
 int lg_launch_shape(const lg_ctx* ctx, int shape[7]);
-/* Recompile the evaluation module for a given shape (LG_ERR_INPUT for an
+/* 1 when the convolution tiles (32 x 64, 8 outputs, paired rows) are split
+ * over clusters of blocks, which the 7 ints do not say: lg_create and the
+ * autotuner choose it for contexts of few tiles. */
+int lg_split_tiles(const lg_ctx* ctx);
+/* Recompile the evaluation module for a given shape, with whole tiles (so a
+ * context with split tiles that is given its own shape back gives them up;
+ * the values are the same) (LG_ERR_INPUT for an
  * invalid one, LG_ERR_UNSUPPORTED when the convolution tile does not fit
  * the device's shared memory). */
 int lg_set_launch_shape(lg_ctx* ctx, const int shape[7]);

@@ -129,6 +129,7 @@ def lib():
         "lg_set_launch_shape": (C.c_int, [vp, ip]),
         "lg_tune_report": (C.c_char_p, [vp]),
         "lg_host_set_active": (C.c_int, [vp]),
+        "lg_split_tiles": (C.c_int, [vp]),
         "lg_tune_candidates": (C.c_int, [C.POINTER(_ImageDesc), C.POINTER(_ObjectDesc), C.c_int,
                                          C.POINTER(_Options), ip, C.c_int]),
         "lg_compile_check_shape": (C.c_int, [C.POINTER(_ImageDesc), C.POINTER(_ObjectDesc), C.c_int,
@@ -437,13 +438,14 @@ def _options(rule, device, max_batch, flags):
     return o
 
 
-def compile_check(width, height, objects, psf=None, rule="g3k7", pcs=None, flags=0):
+def compile_check(width, height, objects, psf=None, rule="g3k7", pcs=None, flags=0, max_batch=0):
     """Compose and compile a model with NVRTC without a GPU; returns the log."""
     psf_a = _f32(psf)
     arr, keep = _objects(objects)
     d = _image_desc(width, height, None, None, psf_a, pcs)
     buf = C.create_string_buffer(1 << 16)
-    rc = lib().lg_compile_check(C.byref(d), arr, len(objects), C.byref(_options(rule, 0, 0, flags)), buf, len(buf))
+    rc = lib().lg_compile_check(C.byref(d), arr, len(objects), C.byref(_options(rule, 0, max_batch, flags)), buf,
+                                len(buf))
     if rc:
         raise LensedError(rc, buf.value.decode(errors="replace"))
     return buf.value.decode(errors="replace")
@@ -607,6 +609,11 @@ class Context:
     def tune_report(self) -> str:
         """The autotuner's candidates and timings ("" if not tuned)."""
         return lib().lg_tune_report(self.h).decode()
+
+    @property
+    def split_tiles(self) -> bool:
+        """Convolution tiles split over clusters of blocks (see lg_split_tiles)."""
+        return bool(lib().lg_split_tiles(self.h))
 
     @property
     def host_set(self) -> bool:

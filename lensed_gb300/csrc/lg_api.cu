@@ -520,7 +520,7 @@ int autotune(lg_ctx* c)
 {
     const lg::Model& m = c->model;
     const lg::Fp mode = ctx_mode(c);
-    const lg::Shape base = choose_shape(m, mode);
+    const lg::Shape base = choose_shape(m, mode, c->max_batch);
     const std::string key = lg::tune_key(lg::compose_source(m, base, mode, lg::Part::EVAL), c->device,
                                          c->max_batch, c->flags & (LG_FLAG_STRICT_FP | LG_FLAG_IEEE_DIV | LG_FLAG_FAST_MATH));
     std::ostringstream rep;
@@ -551,6 +551,8 @@ int autotune(lg_ctx* c)
     std::vector<int> is_render;
     for (const lg::Shape& s : lg::render_candidates(base, mode))
         if (lg::check_shape(s, mode, c->psf, m.psfw).empty()) cand.push_back(s), is_render.push_back(1);
+    // (the quadrature split of a small context's default is not in that table)
+    if (std::find(cand.begin(), cand.end(), base) == cand.end()) cand.push_back(base), is_render.push_back(1);
     if (c->psf)
         for (const lg::Shape& s : lg::conv_candidates(base)) {
             if (!lg::check_shape(s, mode, c->psf, m.psfw).empty()) continue;
@@ -586,7 +588,7 @@ int autotune(lg_ctx* c)
         // the base shape is a render candidate; its convolution time also
         // stands for the base convolution
         const bool base_conv = cand[i].ctx == base.ctx && cand[i].cty == base.cty && cand[i].cr == base.cr &&
-                               cand[i].pair_rows == base.pair_rows;
+                               cand[i].pair_rows == base.pair_rows && cand[i].split_tiles == base.split_tiles;
         if (is_render[i] && r_ms < best_r) best_r = r_ms, br = cand[i];
         if ((!is_render[i] || base_conv) && c->psf && c_ms < best_c) best_c = c_ms, bc = cand[i];
     }
@@ -596,6 +598,7 @@ int autotune(lg_ctx* c)
         chosen.cty = bc.cty;
         chosen.cr = bc.cr;
         chosen.pair_rows = bc.pair_rows;
+        chosen.split_tiles = bc.split_tiles;
     }
     const std::vector<char>* cb = nullptr;
     for (size_t i = 0; i < cand.size(); ++i)
@@ -1111,7 +1114,7 @@ int lg_compile_check(const lg_image_desc* image, const lg_object_desc* objs, int
         const int flags = opts ? opts->flags : 0;
         const lg::Fp mode = lg::fp_mode(flags);
         std::vector<char> cubin;
-        lg::Shape s = choose_shape(m, mode);
+        lg::Shape s = choose_shape(m, mode, opts ? opts->max_batch : 0);
         rc = lg::compile_program(lg::compose_source(m, s, mode, lg::Part::EVAL), lg::fp_fmad(mode), cubin, err,
                                  lg::fp_ieee(flags));
         if (!rc) rc = lg::compile_program(lg::compose_source(m, s, mode, lg::Part::SET), false, cubin, err);
@@ -1426,6 +1429,8 @@ int lg_launch_shape(const lg_ctx* c, int shape[7])
     std::memcpy(shape, v, sizeof v);
     return LG_OK;
 }
+
+int lg_split_tiles(const lg_ctx* c) { return c && c->psf && c->shape.split_tiles ? 1 : 0; }
 
 int lg_set_launch_shape(lg_ctx* c, const int shape[7])
 {

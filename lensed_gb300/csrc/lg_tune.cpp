@@ -11,9 +11,12 @@
 //
 //   render       threads per block (rt), pixels per thread group (rppt) and
 //                the quadrature split (qs: threads of a group sharing its
-//                pixels, each taking every qs-th quadrature point; fast mode
-//                only, since it reorders the quadrature sum);
-//   convolution  output tile (ctx x cty) and outputs per thread (cr).
+//                pixels, each taking every qs-th quadrature point; the fast
+//                mode reorders the quadrature sum with it, the exact mode
+//                gathers the values and keeps the order, the strict mode has
+//                none);
+//   convolution  output tile (ctx x cty), outputs per thread (cr), paired rows,
+//                and for few tiles the paired tile split over a cluster.
 //
 // The two stages are separate kernels, so render candidates are timed with
 // the default convolution and convolution candidates with the default
@@ -44,7 +47,7 @@ std::string Shape::str() const
 {
     std::ostringstream o;
     o << "render " << rt << "x" << rppt << " qs " << qs << ", conv " << ctx << "x" << cty << "/" << cr
-      << (pair_rows ? " paired" : "");
+      << (pair_rows ? " paired" : "") << (split_tiles ? ", split" : "");
     return o.str();
 }
 
@@ -98,11 +101,13 @@ std::vector<Shape> conv_candidates(const Shape& base, bool multi)
     for (int i = 0; i < n; ++i) {
         const int* c = multi ? units[i] : base.pair_rows ? paired[i] : single[i];
         Shape s = base;
+        s.split_tiles = false;
         s.ctx = c[0];
         s.cty = c[1];
         s.cr = c[2];
         out.push_back(s);
     }
+    if (base.split_tiles) out.push_back(base);
     if (!multi && base.pair_rows) {
         // single-row tiles of two or four outputs per thread: the most
         // threads for a batch of one or a few candidates (same per-pixel
@@ -114,6 +119,7 @@ std::vector<Shape> conv_candidates(const Shape& base, bool multi)
             s.cty = c[1];
             s.cr = c[2];
             s.pair_rows = false;
+            s.split_tiles = false;
             out.push_back(s);
         }
     }
@@ -133,6 +139,8 @@ std::string check_shape(const Shape& s, Fp mode, bool psf, int psfw)
     if (s.cr != 2 && s.cr != 4 && s.cr != 8 && s.cr != 16) return "convolution outputs per thread must be 2, 4, 8 or 16";
     if (s.ctx < s.cr || s.ctx % s.cr || s.ctx > 256) return "convolution tile width must be a multiple of cr";
     if (s.pair_rows && (strict || psfw > 49)) return "paired rows need the fast or exact mode and a PSF up to 49 wide";
+    if (s.split_tiles && !(s.pair_rows && s.ctx == 32 && s.cty == 64 && s.cr == 8))
+        return "split tiles are paired ones of 32 x 64 with 8 outputs";
     if (s.pair_rows && (s.cr % 8 || s.cty % 2)) return "paired rows need cr % 8 == 0 and an even tile height";
     if (s.cty < 1 || s.cty > 256) return "convolution tile height must be in [1, 256]";
     const int threads = (s.ctx / s.cr) * s.conv_block_y();
@@ -179,9 +187,10 @@ void load_cache_file()
         std::istringstream is(line);
         std::string key;
         Shape s;
-        int pr = 0;
+        int pr = 0, split = 0;
         if (is >> key >> s.rt >> s.rppt >> s.qs >> s.ctx >> s.cty >> s.cr >> pr) {
             s.pair_rows = pr != 0;
+            s.split_tiles = is >> split && split != 0;  // (lines without it: whole tiles)
             g_cache[key] = s;
         }
     }
@@ -233,8 +242,8 @@ void tune_cache_put(const std::string& key, const Shape& s)
     g_cache[key] = s;
     if (const char* p = cache_path()) {
         if (FILE* f = std::fopen(p, "a")) {
-            std::fprintf(f, "%s %d %d %d %d %d %d %d\n", key.c_str(), s.rt, s.rppt, s.qs, s.ctx, s.cty, s.cr,
-                         s.pair_rows ? 1 : 0);
+            std::fprintf(f, "%s %d %d %d %d %d %d %d%s\n", key.c_str(), s.rt, s.rppt, s.qs, s.ctx, s.cty, s.cr,
+                         s.pair_rows ? 1 : 0, s.split_tiles ? " 1" : "");
             std::fclose(f);
         }
     }
