@@ -29,7 +29,9 @@ def layout(d, layers, width, hidden):
     return out, off
 
 
-def loss_grad(params, x, d, layers, width, hidden):
+def loss_grad(params, x, d, layers, width, hidden, act=lambda a: a):
+    """Loss and gradient; act rounds the hidden activations as they are stored
+    (bf16 for the training step with BF16 activations)."""
     L, n = layout(d, layers, width, hidden)
     p = np.asarray(params, np.float64)
     M = x.shape[0]
@@ -43,7 +45,7 @@ def loss_grad(params, x, d, layers, width, hidden):
         for k, (w0, kin, kout, b) in enumerate(dense):
             W = p[w0:w0 + kin * kout].reshape(kin, kout)
             z = acts[-1] @ W + p[b:b + kout]
-            acts.append(np.maximum(z, 0) if k < len(dense) - 1 else z)
+            acts.append(act(np.maximum(z, 0)) if k < len(dense) - 1 else z)
         o = acts[-1]
         sr, t = o[:, :db], o[:, db:]
         s = CLAMP * np.tanh(sr / CLAMP)
