@@ -520,7 +520,7 @@ int autotune(lg_ctx* c)
 {
     const lg::Model& m = c->model;
     const lg::Fp mode = ctx_mode(c);
-    const lg::Shape base = choose_shape(m, mode, c->max_batch);
+    const lg::Shape base = choose_shape(m, mode), few = choose_shape(m, mode, c->max_batch);
     const std::string key = lg::tune_key(lg::compose_source(m, base, mode, lg::Part::EVAL), c->device,
                                          c->max_batch, c->flags & (LG_FLAG_STRICT_FP | LG_FLAG_IEEE_DIV | LG_FLAG_FAST_MATH));
     std::ostringstream rep;
@@ -535,9 +535,9 @@ int autotune(lg_ctx* c)
     for (size_t i = 0; i < m.pars.size(); ++i)
         if (!m.pars[i].has_prior) {
             std::vector<char> cubin;
-            if ((rc = compile_eval(c, base, cubin)) || (rc = load_eval(c, base, cubin))) return rc;
+            if ((rc = compile_eval(c, few, cubin)) || (rc = load_eval(c, few, cubin))) return rc;
             c->tune_report = "not tuned (no prior for " + m.pars[i].id + " to draw candidates from): " +
-                             base.str() + "\n";
+                             few.str() + "\n";
             return LG_OK;
         }
     const int B = c->max_batch;
@@ -546,15 +546,21 @@ int autotune(lg_ctx* c)
     if ((rc = c->cuda(cudaMemcpy(c->d_params, c->h_params, (size_t)B * np * 8, cudaMemcpyHostToDevice), "params")))
         return rc;
     // render candidates with the base convolution, convolution candidates
-    // with the base render
+    // with the base render; the default of a context for few candidates (its
+    // quadrature split, its split tiles) beside the shapes around the default
+    // for many
     std::vector<lg::Shape> cand;
     std::vector<int> is_render;
     for (const lg::Shape& s : lg::render_candidates(base, mode))
         if (lg::check_shape(s, mode, c->psf, m.psfw).empty()) cand.push_back(s), is_render.push_back(1);
-    // (the quadrature split of a small context's default is not in that table)
-    if (std::find(cand.begin(), cand.end(), base) == cand.end()) cand.push_back(base), is_render.push_back(1);
+    lg::Shape extra = base;
+    extra.rt = few.rt;
+    extra.qs = few.qs;
+    if (std::find(cand.begin(), cand.end(), extra) == cand.end()) cand.push_back(extra), is_render.push_back(1);
+    extra = base;
+    extra.split_tiles = few.split_tiles;
     if (c->psf)
-        for (const lg::Shape& s : lg::conv_candidates(base)) {
+        for (const lg::Shape& s : lg::conv_candidates(extra)) {
             if (!lg::check_shape(s, mode, c->psf, m.psfw).empty()) continue;
             bool dup = false;
             for (const lg::Shape& t : cand) dup = dup || t == s;

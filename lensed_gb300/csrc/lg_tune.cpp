@@ -107,7 +107,6 @@ std::vector<Shape> conv_candidates(const Shape& base, bool multi)
         s.cr = c[2];
         out.push_back(s);
     }
-    if (base.split_tiles) out.push_back(base);
     if (!multi && base.pair_rows) {
         // single-row tiles of two or four outputs per thread: the most
         // threads for a batch of one or a few candidates (same per-pixel
@@ -123,6 +122,7 @@ std::vector<Shape> conv_candidates(const Shape& base, bool multi)
             out.push_back(s);
         }
     }
+    if (base.split_tiles) out.push_back(base);
     return out;
 }
 
