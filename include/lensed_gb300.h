@@ -129,7 +129,7 @@ typedef struct {
                        * time is served faster by a context of its own with
                        * max_batch = 1; its program is another one than a batch
                        * context's of the same model, and the first of each in
-                       * a process is compiled (about half a second). */
+                       * a process is compiled (about a second). */
     int flags;        /* LG_FLAG_* */
 } lg_options;
 
@@ -280,10 +280,11 @@ int lg_eval_profile(lg_ctx* ctx, const double* d_params, int B, double* d_logL, 
  * work-group size and halves the convolution tile until it fits local
  * memory.  With LG_FLAG_AUTOTUNE, lg_create compiles candidate shapes in
  * parallel, times them on max_batch candidates drawn from the priors and
- * keeps the fastest render and convolution; the choice is cached per
- * program, device, batch and flags in the process, and in the text file
- * named by the environment variable LG_TUNE_CACHE when it is set.  Results
- * are the same for every shape up to the order of FP64 partial sums, and,
+ * keeps the fastest render and convolution (for a context of few convolution
+ * tiles split ones among them); the choice is cached per program, device,
+ * batch and flags in the process, and in the text file named by the
+ * environment variable LG_TUNE_CACHE when it is set.  Results are the same
+ * for every shape up to the order of FP64 partial sums, and, in the fast mode
  * with a quadrature split above 1, of the FP32 quadrature sum. */
 int lg_launch_shape(const lg_ctx* ctx, int shape[7]);
 /* 1 when the convolution tiles (32 x 64, 8 outputs, paired rows) are split

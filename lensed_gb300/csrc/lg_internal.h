@@ -186,9 +186,19 @@ bool crf_in_smem(const Shape& s, Fp mode);
 
 // A context whose largest batch has at most kSplitTiles convolution tiles
 // splits each over a cluster of 8 blocks: 608 blocks then fill 152 SMs.
-// Convolution stage, whole against split tiles (us): 256^2, 25^2 PSF, 32 tiles
-// 22.5 / 16.3, 64 tiles 24.5 / 20.5, 128 tiles 22.5 / 28.7; 64^2, 17^2 PSF, 32
-// tiles 20.4 / 12.2, 64 tiles 20.5 / 16.4, 128 tiles 20.4 / 20.4.
+// Convolution stage with whole tiles / split ones / single rows of 32 x 16 with
+// 4 outputs, the tuner's other candidate for small batches (us, in steps of 2):
+//   tiles        PSF 5^2            17^2               25^2               49^2
+//   8  (1 of 101 x 77)  12.3/9.2/10.2  18.4/12.3/14.3  22.5/15.3/14.3  57.3/20.5/32.8
+//   32 (1 of 256^2)    12.3/10.2/10.2  20.5/12.3/14.3  24.5/16.4/16.4  59.4/26.6/32.8
+//   56 (7 of 101 x 77) 12.3/10.2/10.2  20.1/14.3/14.3  22.5/20.5/14.3  59.4/43.0/30.7
+//   64 (2 of 256^2)    14.3/10.2/12.3  20.5/16.4/16.4  24.5/22.3/18.4  59.4/43.0/38.9
+//   76 (38 of 64^2)    12.4/12.3/10.2  20.5/16.4/16.4  22.5/24.6/16.4  57.4/53.2/36.9
+// and at 128 tiles whole ones win (25^2: 22.5 against 28.7).  So above 32 tiles
+// with a wide PSF the single rows are faster still (a call of 7 candidates of
+// 101 x 77 with a 49^2 PSF: 99.0 / 84.2 / 71.0), but they group the FP64 sums of
+// chi^2 otherwise, and logL's last bits would then depend on the batch size a
+// context was made for; they are left to the tuner.
 // With a split quadrature while the threads stay below kSplitRays (1024 an
 // SM), render stage, unsplit / 2 / 4 threads (us): 256^2, 25 points, 1
 // candidate 40.4 / 30.2 / 28.1, 2 candidates 48.7 / 46.6 / 46.6, 4 candidates
@@ -211,8 +221,9 @@ int compile_program(const std::string& src, bool fmad, std::vector<char>& cubin,
 
 // ---------------------------------------------------------------- autotuner
 // Candidate launch shapes around a base shape (lg_tune.cpp): render shapes
-// vary threads, pixels per group and (fast mode) the quadrature split;
-// convolution shapes vary the tile and outputs per thread.
+// vary threads, pixels per group and (fast and exact modes) the quadrature
+// split; convolution shapes vary the tile, outputs per thread, paired rows and,
+// around a base that splits its tiles, the split.
 std::vector<Shape> render_candidates(const Shape& base, Fp mode);
 std::vector<Shape> conv_candidates(const Shape& base, bool multi = false);
 // "" when the shape is valid for the program, else the reason.

@@ -67,7 +67,7 @@ void emit_compute(std::ostringstream& o, const Model& m)
 }
 
 // The same sum for two rays at once (lg_pair2), for the paired ray kernels
-// of the fast mode: plugins with template evaluation functions are called
+// of the fast and exact modes: plugins with template evaluation functions are called
 // with the pair; any other plugin is called once per ray.
 void emit_compute2(std::ostringstream& o, const Model& m, Fp mode)
 {

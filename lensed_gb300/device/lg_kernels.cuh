@@ -106,13 +106,14 @@ LG_DEV void lg_tile_done(double s, double* __restrict__ partials, int ntiles, in
 // kernel/lensed.cl:9-39.  Block (tile, candidate), or in the exact modules
 // (tile, `per` candidates one after the other: the tables of the correctly
 // rounded functions are copied to shared memory once for all of them); each
-// group of LG_QS threads integrates LG_RPPT pixels over the quadrature rule: strided by the
-// group count in the scalar kernel (so that loads and stores coalesce),
-// adjacent in the paired kernel (a thread's two rays are neighbours, so they
-// mostly take the same branches; stores are float2).  With LG_QS > 1 the
-// threads of a group take quadrature points n = sub, sub + LG_QS, ... and
-// their sums are combined by a butterfly of shuffles (every lane ends with
-// the same, order-independent result).  MODE 0 stores the raw model, MODE 1
+// group of LG_QS threads integrates LG_RPPT pixels over the quadrature rule:
+// strided by the group count in the scalar kernel (so that loads and stores
+// coalesce), adjacent in the paired kernel (a thread's two rays are
+// neighbours, so they mostly take the same branches; stores are float2).  With
+// LG_QS > 1 the threads of a group take quadrature points n = sub, sub + LG_QS,
+// ...; in the fast mode their sums are combined by a butterfly of shuffles
+// (every lane ends with the same, order-independent result), in the exact mode
+// their values are summed in the rule's order.  MODE 0 stores the raw model, MODE 1
 // reduces the chi^2 directly (no PSF), MODE 2 stores value and error for one
 // candidate.
 #if defined(LG_PAIRED) && LG_RPPT % 2 == 0
@@ -148,8 +149,8 @@ LG_DEV void lg_render_tile(const lg_model* __restrict__ models, float* __restric
         e[j] = 0.0f;
     }
 #if defined(LG_PAIRED) && LG_RPPT % 2 == 0
-    // the fast mode traces the thread's pixels two at a time with paired
-    // FP32 instructions; each lane computes what the scalar loop computes
+    // the fast and exact modes trace the thread's pixels two at a time with
+    // paired FP32 instructions; each lane computes what the scalar loop computes
     lg_pair px[LG_RPPT / 2], py[LG_RPPT / 2], pv[LG_RPPT / 2], pe[LG_RPPT / 2];
 #pragma unroll
     for (int j = 0; j < LG_RPPT / 2; ++j) {

@@ -17,7 +17,7 @@
 #ifndef LG_RPPT
 #define LG_RPPT 2
 #endif
-// quadrature split (fast mode only), as in the single-system render kernel
+// quadrature split, as in the single-system render kernel
 #ifndef LG_QS
 #define LG_QS 1
 #endif
@@ -312,7 +312,7 @@ LG_DEV double lg_multi_conv_unit(const float* __restrict__ src, const float* __r
 }
 
 #if defined(LG_PAIRED)
-// The paired-row unit of the fast mode for PSFs up to 49 pixels wide: a
+// The paired-row unit of the fast and exact modes for PSFs up to 49 pixels wide: a
 // 32 x (2 LG_CTY) output tile, each thread LG_CR columns of rows y and
 // y + LG_CTY, in the layout, order and partial-sum grouping of the
 // single-system kernel (so each system's logL is identical to its own
