@@ -1103,17 +1103,17 @@ LG_CRF_DEV float lg_crf_atan2(float y, float x)
 
 #ifndef LG_CRF_NO_QUICK
 // ------------------------------------------- quick phases of the EPL lens --
-// x^y for one exponent: ln x = s1 + a from the quick log (a its float part),
-// t = y ln x as a double word (y s1 exactly, y a added, a two-sum), e^t as in
-// lg_crf_exp with the low part added to the reduction's.  |a| is at most 1.135
-// 2^-10 (r, and e ln2_lo up to 2^-12.9), so in units of 2^-34: a's rounding 1,
-// those of (e - 1/2) ln2_lo + Ll, of t and of its shift back by D 1/8 each,
-// ln2_lo's own 0.09 (1.46 in all; 1.455 is met), the rounding of y a + (the
-// product's error) 1.14 |y|, and the square of t's low part, which the exp
-// leaves out, 0.125 |y| (2^-37, for |t| above 64 only, so |y| above 1).  A
-// power is below 2 times its exp's scale: 2 (1.46 + 1.14 + 0.125) |y| 2^-34 =
-// 1.36 |y| 2^-32, and the interval of the exp is widened by 1.5 |y| 2^-32 each
-// way.  x in the log's range with |t| <= 86; the rest, and undecided
+// x^y for one exponent: ln x = s1 + r + t from the quick log, T = y ln x as a
+// double word (y s1 exactly, y t and y r added, a two-sum), e^T as in
+// lg_crf_exp with the low part added to the reduction's.  Error of T in units
+// of 2^-34 |y|: the roundings of (e - 1/2) ln2_lo + Ll, of t, of its shift back
+// by D and of y t added to the product's error 1/8 each (t stays below 2^-12.8),
+// ln2_lo's own 0.09, the rounding of y r added to that 1.14 (a sum up to 1.14
+// 2^-10 |y|); the square of T's low part, which the exp leaves out, 0.14 (2^-37,
+// for |T| above 64 only, so |y| above 1): 1.9 in all.  A power is below 2 times
+// its exp's scale, so that is 0.95 2^-32 |y|, and the interval of the exp is
+// widened by 2^-32 |y| each way.  (r and t summed to a float first were 1
+// more.)  x in the log's range with |T| <= 86; the rest, and undecided
 // roundings, in the full phase.
 LG_CRF_COLD float crf_rest_pow(float x, float y) { LG_CRF_REST_COUNT(); return lg_crf_pow(x, y); }
 template <class F>
@@ -1121,10 +1121,9 @@ LG_CRF_DEV F lg_crf_pow1(F x, float y)
 {
     F s1, r, t, e;
     crf_quick_log(x, s1, r, t, e);
-    const F a = crf_add(r, crf_add(t, crf_bc<F>(-0x1.6p-34f)));
     const F Y = crf_bc<F>(y);
     const F ph = crf_mul(Y, s1);
-    const F pl = crf_fma(Y, a, crf_fma(Y, s1, crf_neg(ph)));
+    const F pl = crf_fma(Y, r, crf_fma(Y, crf_add(t, crf_bc<F>(-0x1.6p-34f)), crf_fma(Y, s1, crf_neg(ph))));
     const F T = crf_add(ph, pl);  // two-sum
     const F bb = crf_sub(T, ph);
     const F Tl = crf_add(crf_sub(ph, crf_sub(T, bb)), crf_sub(pl, bb));
@@ -1140,7 +1139,7 @@ LG_CRF_DEV F lg_crf_pow1(F x, float y)
         crf_set(th, i, E.x);
         crf_set(tl, i, E.y);
     }
-    const float wide = crf_mul(crf_fabsf(y), 0x1.8p-32f);
+    const float wide = crf_mul(crf_fabsf(y), 0x1p-32f);
     const F c = crf_fma(th, rh, crf_add(crf_fma(th, sm, crf_fma(tl, rh, tl)), crf_bc<F>(wide)));
     const F z = crf_add(th, c);
     const F rem = crf_sub(c, crf_sub(z, th));

@@ -1,5 +1,5 @@
 // Host harness for lg_crf_pow1 where its error is largest: bases whose quick
-// logarithm is furthest off, exponents whose result lies just below a power
+// logarithm's float part is furthest off, exponents whose result lies just below a power
 // of two (there the error counts most against the rounding), and the
 // arguments given on the command line.
 //   crf_pow <bases> <seed> [<x> <y>]...

@@ -1,6 +1,7 @@
 """The exact modules' paired power (lg_crf_pow1) on the CPU where its error is
 largest: equal to the double evaluation rounded once, bit for bit.  The first
-power is one whose rounding an interval of 2^-32 |y| decides wrongly."""
+power is one whose rounding an interval of 2^-32 |y| decides wrongly when the
+logarithm's r and t are summed to a float before y times it is taken."""
 import os
 import subprocess
 
